@@ -24,7 +24,7 @@ FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", 
          "--expt-relaxed-constexpr", "-I", CSRC, "-I", os.path.join(ROOT, "include")]
 
 UNITS = [
-    ("setup.cu", []), ("eigen.cu", []), ("layout.cu", []), ("precond.cu", []),
+    ("setup.cu", []), ("eigen.cu", []), ("fixed_tab.cu", []), ("layout.cu", []), ("precond.cu", []),
     ("operator.cu", []), ("mg.cu", []), ("diag.cu", []), ("stream3d.cu", []), ("mapped.cu", []), ("mapped_mf.cu", []), ("local.cu", []), ("mlp.cu", []), ("learned.cu", []), ("c0ip.cu", []),
     ("plane_inst.cu", ["-DPLANE_BZ=8"]), ("plane_inst.cu", ["-DPLANE_BZ=4"]),
     ("stream_k5.cu", ["-DK5_PART=0"]), ("stream_k5.cu", ["-DK5_PART=1"]),

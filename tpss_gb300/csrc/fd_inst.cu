@@ -1,6 +1,9 @@
 // fd_inst.cu -- instantiations of the fused Schwarz color kernel for one arithmetic type and
 // dimension.  Compiled once per (FD_T, FD_DIM) pair (float/double x 2/3), so the four
 // translation units build in parallel.
+#include <type_traits>
+
+#include "fd_fixed.cuh"
 #include "fd_kernels.cuh"
 #include "internal.h"
 
@@ -17,6 +20,37 @@
 
 namespace tpss
 {
+namespace
+{
+// FP64: the contractions run on the integer pipe (fd_fixed.cuh)
+template<typename T, int DIM, int NCP, int K1>
+bool launch_one(const fd::KernelArgs &a, const FdLaunch &l, cudaStream_t s, int sms)
+{
+  if constexpr(std::is_same_v<T, double>)
+  {
+    fd::FixArgs f;
+    f.k = a;
+    f.fix = l.fix;
+    f.fix_eo = l.fix_eo;
+    f.fexp = l.fexp;
+    f.fexp_eo = l.fexp_eo;
+    f.fp64_only = l.fp64_only;
+    return fd::launch_fixed<DIM, NCP, K1>(f, s, sms, l.variant);
+  }
+  else
+    return fd::launch<T, DIM, NCP, K1>(a, s, sms, l.variant);
+}
+
+template<typename T, int DIM, int NCP, int K1>
+constexpr int variants()
+{
+  if constexpr(std::is_same_v<T, double>)
+    return fd::FixCfg<DIM, NCP, K1>::n_variants();
+  else
+    return fd::Cfg<T, DIM, NCP, K1>::n_variants();
+}
+}  // namespace
+
 bool TPSS_FD_FN(int k, int ncp, const FdLaunch &l, cudaStream_t s)
 {
   fd::KernelArgs a;
@@ -38,7 +72,7 @@ bool TPSS_FD_FN(int k, int ncp, const FdLaunch &l, cudaStream_t s)
   a.keep_class = l.keep_class;
   const int sms = num_sms();
 #define TPSS_FD_CASE(NCP, K1) \
-  if(ncp == NCP && k + 1 == K1) return fd::launch<FD_T, FD_DIM, NCP, K1>(a, s, sms, l.variant);
+  if(ncp == NCP && k + 1 == K1) return launch_one<FD_T, FD_DIM, NCP, K1>(a, l, s, sms);
   TPSS_FD_CASE(1, 2) TPSS_FD_CASE(1, 3) TPSS_FD_CASE(1, 4) TPSS_FD_CASE(1, 5)
   TPSS_FD_CASE(1, 6) TPSS_FD_CASE(1, 7) TPSS_FD_CASE(1, 8)
   TPSS_FD_CASE(2, 2) TPSS_FD_CASE(2, 3) TPSS_FD_CASE(2, 4) TPSS_FD_CASE(2, 5)
@@ -51,7 +85,7 @@ bool TPSS_FD_FN(int k, int ncp, const FdLaunch &l, cudaStream_t s)
 int TPSS_CAT(TPSS_CAT(fd_variants_, FD_T), TPSS_CAT(_, FD_DIM))(int k, int ncp)
 {
 #define TPSS_FD_CASE(NCP, K1) \
-  if(ncp == NCP && k + 1 == K1) return fd::Cfg<FD_T, FD_DIM, NCP, K1>::n_variants();
+  if(ncp == NCP && k + 1 == K1) return variants<FD_T, FD_DIM, NCP, K1>();
   TPSS_FD_CASE(1, 2) TPSS_FD_CASE(1, 3) TPSS_FD_CASE(1, 4) TPSS_FD_CASE(1, 5)
   TPSS_FD_CASE(1, 6) TPSS_FD_CASE(1, 7) TPSS_FD_CASE(1, 8)
   TPSS_FD_CASE(2, 2) TPSS_FD_CASE(2, 3) TPSS_FD_CASE(2, 4) TPSS_FD_CASE(2, 5)

@@ -1,0 +1,166 @@
+// fixed64.cuh -- 64-bit contractions on the integer pipe.
+//
+// GB300 issues 2 FP64 multiply-adds per clock and SM but 27 32 x 32 + 64 bit integer ones
+// (IMAD.WIDE; both measured on all SMs in 5 x 5 pairs of contractions, the pipe's limit is 32), and
+// three of these do the product of an FP64 multiply-add to 58 bits: 17.6 clocks per warp and value
+// of such a contraction against 81. The kernels that include this file keep the values of a block (a patch, a
+// cell) as 64-bit integers with one exponent per block (block floating point):
+//   value = x 2^e,  |x| < 2^59,  coefficient = c 2^-F,  sum_j |c_ij| <= 2^62 in every row i.
+// With signed 32-bit limbs x = xh 2^32 + xl, c = ch 2^32 + cl (xl, cl in [-2^31, 2^31)) a row's
+// sum is  sum_j c_ij x_j / 2^64 = sum ch xh + (sum ch xl + cl xh) / 2^32 + (cl xl, dropped):
+// three IMAD.WIDE per product, the dropped terms and the rounding stay below one unit 2^(e+64-F),
+// and the accumulators cannot overflow (|sum ch xh| < 2^60, |sum ch xl + cl xh| < 2^63 for up to
+// 16 terms).  After every contraction the block is shifted up again to 59 bits by the headroom
+// its largest value leaves, so one contraction's error is 2^-58 of (row sum of |c|) x (largest
+// |x| of the block), where an FP64 chain makes up to 2^-53 sum_j |c_ij x_j| per addition.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+namespace tpss
+{
+namespace fx
+{
+// 64-bit accumulator of 32 x 32-bit products. add() is one IMAD.WIDE: it is written with the carry
+// flag because ptxas splits the accumulation of mad.wide chains into products and separate 64-bit
+// additions (43 instead of 30 instructions per value of a 5 x 5 pair of contractions, 19.6 instead of
+// 17.6 clocks per warp)
+struct Acc
+{
+  unsigned lo;
+  int hi;
+  __device__ __forceinline__ explicit Acc(unsigned l = 0) : lo(l), hi(0) {}
+  __device__ __forceinline__ void add(int a, int b)
+  {
+    asm("mad.lo.cc.u32 %0, %2, %3, %0;\n\tmadc.hi.s32 %1, %2, %3, %1;" : "+r"(lo), "+r"(hi) : "r"(a), "r"(b));
+  }
+  // the first product of a sum (from a zero accumulator add() would be two instructions)
+  __device__ __forceinline__ void start(int a, int b)
+  {
+    asm("{.reg .b64 t;\n\tmul.wide.s32 t, %2, %3;\n\tmov.b64 {%0, %1}, t;}" : "=r"(lo), "=r"(hi) : "r"(a), "r"(b));
+  }
+  __device__ __forceinline__ int64_t value() const { return (int64_t)((uint64_t)(unsigned)hi << 32 | lo); }
+};
+
+__device__ __forceinline__ int hi32(int64_t x) { return (int)(x >> 32); }
+
+// signed limbs of x
+__device__ __forceinline__ void split(int64_t x, int &h, int &l)
+{
+  l = (int)x;
+  h = (int)(x >> 32) + (int)((unsigned)l >> 31);
+}
+
+// x >> s and x << s with s >= 64 giving 0 (or the sign): PTX clamps the amounts
+__device__ __forceinline__ uint64_t shr_u(uint64_t x, int s)
+{
+  uint64_t r;
+  asm("shr.u64 %0, %1, %2;" : "=l"(r) : "l"(x), "r"(s));
+  return r;
+}
+__device__ __forceinline__ int64_t shr_s(int64_t x, int s)
+{
+  int64_t r;
+  asm("shr.s64 %0, %1, %2;" : "=l"(r) : "l"(x), "r"(s));
+  return r;
+}
+__device__ __forceinline__ int64_t shl(int64_t x, int s)
+{
+  int64_t r;
+  asm("shl.b64 %0, %1, %2;" : "=l"(r) : "l"(x), "r"(s));
+  return r;
+}
+// x 2^s for either sign of s (|x| 2^s must fit)
+__device__ __forceinline__ int64_t shift(int64_t x, int s) { return shr_s(shl(x, max(s, 0)), max(-s, 0)); }
+
+// bits of |x| in the high word (|x| or |x| - 1): ORed over a block, their highest set bit gives the
+// block's headroom
+__device__ __forceinline__ unsigned mag_hi(int64_t x)
+{
+  const int h = (int)(x >> 32);
+  return (unsigned)(h ^ (h >> 31));
+}
+
+// shift that brings a block whose high-word magnitudes OR to m (< 2^27) to 59 bits
+__device__ __forceinline__ int headroom(unsigned m) { return __clz(m | 1u) - 5; }
+
+// double -> integer with unit 2^(emax - 1023 - 58), emax the block's largest biased exponent
+// (truncated toward zero beyond the 59 bits; zeros and denormals give 0 for emax >= 64)
+__device__ __forceinline__ int64_t from_double(double v, int emax)
+{
+  const int hi = __double2hiint(v);
+  const unsigned lo = (unsigned)__double2loint(v);
+  const unsigned mh = ((unsigned)hi & 0xfffffu) | 0x100000u;
+  const int e = (int)(((unsigned)hi >> 20) & 0x7ffu);
+  const uint64_t m = (((uint64_t)mh << 32) | lo) << 6;
+  const int64_t a = (int64_t)shr_u(m, emax - e);
+  const int64_t s = (int64_t)(hi >> 31);
+  return (a ^ s) - s;
+}
+
+// 2^e as a double, e in [-1022, 1023]
+__device__ __forceinline__ double pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }
+
+// positive normal double r = m 2^q with 2^60 <= m < 2^61, m in signed limbs
+__device__ __forceinline__ void split_positive(double r, int &mh, int &ml, int &q)
+{
+  const int hi = __double2hiint(r);
+  const unsigned lo = (unsigned)__double2loint(r);
+  const uint64_t m = (((uint64_t)(((unsigned)hi & 0xfffffu) | 0x100000u) << 32) | lo) << 8;
+  split((int64_t)m, mh, ml);
+  q = (int)((unsigned)hi >> 20) - 1023 - 60;
+}
+
+// x m / 2^61 (|x| < 2^60, m as above): |result| <= |x|, error below 3 units
+__device__ __forceinline__ int64_t mul_m61(int64_t x, int mh, int ml)
+{
+  int xh, xl;
+  split(x, xh, xl);
+  Acc M(1u << 28), S;
+  M.add(xl, mh);
+  M.add(xh, ml);
+  S.start(xh, mh);
+  return (S.value() << 3) + (M.value() >> 29);
+}
+
+// ---- coefficient rows: int2 (x: low limb, y: high limb), read as pairs
+// y[p] = sum_j c_j x_j / 2^64 of one row of H coefficients for P vectors x in limbs
+template<int H, int P>
+__device__ __forceinline__ void row_dot(const int2 *__restrict__ row, const int (&xh)[P][H], const int (&xl)[P][H],
+                                        int64_t (&y)[P])
+{
+  Acc M[P], S[P];
+#pragma unroll
+  for(int p = 0; p < P; ++p) M[p] = Acc(1u << 31);
+  const int4 *row4 = reinterpret_cast<const int4 *>(row);
+#pragma unroll
+  for(int j2 = 0; j2 < (H + 1) / 2; ++j2)
+  {
+    const int4 c = row4[j2];
+#pragma unroll
+    for(int p = 0; p < P; ++p)
+    {
+      M[p].add(c.y, xl[p][2 * j2]);
+      M[p].add(c.x, xh[p][2 * j2]);
+      if(j2 == 0) S[p].start(c.y, xh[p][0]);
+      else S[p].add(c.y, xh[p][2 * j2]);
+    }
+    if(2 * j2 + 1 < H)
+    {
+      const int j = 2 * j2 + 1 < H ? 2 * j2 + 1 : 0;
+#pragma unroll
+      for(int p = 0; p < P; ++p)
+      {
+        M[p].add(c.w, xl[p][j]);
+        M[p].add(c.z, xh[p][j]);
+        S[p].add(c.w, xh[p][j]);
+      }
+    }
+  }
+#pragma unroll
+  for(int p = 0; p < P; ++p) y[p] = S[p].value() + M[p].hi;
+}
+}  // namespace fx
+}  // namespace tpss

@@ -258,6 +258,11 @@ struct FdTables
   DeviceBuffer<double> fd64_eo;  // the same in FP64 (per-color kernel, FP64 smoother)
   DeviceBuffer<int32_t> sym;
   bool has_eo = false;           // some entry has the even/odd form
+  // FP64 smoother on the integer pipe (fd_fixed.cuh): the coefficients of fd64 and fd64_eo as 64-bit
+  // integers c 2^F in signed 32-bit limbs, same strides (the eigenvalue words unused), and per
+  // entry F of S^T and of S
+  DeviceBuffer<int2> fix64, fix64_eo, fexp, fexp_eo;
+  bool fix_ok = false;           // finite tables and positive eigenvalue sums: the integers apply
   // eigenvalues of every entry in the order the kernels read them (the even/odd order for
   // mirror-symmetric entries), n_entries x n, host
   std::vector<double> lam_kernel;
@@ -373,6 +378,9 @@ struct FdLaunch
   const unsigned char *keep_mask = nullptr;  // RAS boolean weights (FdTables::keep_mask) or nullptr
   const int32_t *keep_class = nullptr;       // first patch of the range
   int variant = 0;                           // work decomposition (patches per CTA) of the autotuner
+  // FP64 only: integer forms of fd and fd_eo and their scales (FdTables::fix*)
+  const int2 *fix = nullptr, *fix_eo = nullptr, *fexp = nullptr, *fexp_eo = nullptr;
+  bool fp64_only = false;
 };
 bool launch_fd_f32(int dim, int k, int ncp, const FdLaunch &a, cudaStream_t s);
 bool launch_fd_f64(int dim, int k, int ncp, const FdLaunch &a, cudaStream_t s);
@@ -395,6 +403,8 @@ bool mapped_apply_mf(const tpss_operator &op, double *dst, const double *src, cu
 // its FP32 arithmetic (FP32 copies of the cell blocks, face geometry and source; FP64 result)
 bool mapped_apply_mf_f32(tpss_operator &op, double *dst, const double *src, cudaStream_t s,
                          const double *rhs = nullptr);
+// integer forms of the FP64 tables (fixed_tab.cu)
+void build_fixed_tables(FdTables &T);
 // FD setup helpers (precond.cu, eigen.cu)
 void gen_eig_batched(int n, int n_problems, const std::vector<double> &Ms,
                      const std::vector<double> &As, std::vector<double> &S,

@@ -8,6 +8,7 @@
 // (additive_schwarz_operation, templates:665-688); multiplicative = residual update with the
 // level operator between colors in the color sequence of get_color_sequence
 // (schwarz_preconditioner.h:532-567, templates:691-732).
+#include <algorithm>
 #include <chrono>
 #include <cmath>
 #include <cstring>
@@ -143,6 +144,34 @@ void build_reciprocals(const tpss_layout &L, FdTables &T)
   T.rcp_E = E;
 }
 
+// The integer form of the FP64 smoother needs finite eigenvectors and positive eigenvalue sums in
+// every patch (an ip_factor too small for coercivity gives neither); otherwise its kernel runs the
+// FP64 passes.
+bool fixed_applies(const tpss_layout &L, const FdTables &T, bool keyed)
+{
+  const int n = L.n, dim = L.dim;
+  for(double v : T.S_host)
+    if(!(std::fabs(v) < 1e30)) return false;
+  std::vector<double> lo(T.n_entries), hi(T.n_entries);
+  bool positive = true;
+  for(int e = 0; e < T.n_entries; ++e)
+  {
+    const auto mm = std::minmax_element(&T.lam_host[(size_t)e * n], &T.lam_host[(size_t)e * n] + n);
+    lo[e] = *mm.first;
+    hi[e] = *mm.second;
+    if(!(std::fabs(lo[e]) < 1e60 && std::fabs(hi[e]) < 1e60)) return false;
+    positive = positive && lo[e] > 1e-60;
+  }
+  if(positive) return true;
+  for(int64_t p = 0; p < L.P; ++p)
+  {
+    double sum = 0.0;
+    for(int d = 0; d < dim; ++d) sum += lo[keyed ? L.patch_fd_key[(size_t)p * dim + d] : p * dim + d];
+    if(!(sum > 1e-60)) return false;
+  }
+  return true;
+}
+
 }  // namespace
 
 // 1-D patch matrices (mass, SIPG Laplace) of every FD key of the layout
@@ -268,6 +297,8 @@ std::shared_ptr<FdTables> build_tables(const tpss_layout &L, Penalty ip, bool ra
   T->fd32.upload(t32.data(), t32.size());
   build_even_odd(L, *T, Ms, As, keyed);
   if(keyed) build_reciprocals(L, *T);
+  build_fixed_tables(*T);
+  T->fix_ok = fixed_applies(L, *T, keyed);
   if(ras)
   {
     // RAS weights: 1 / (number of patches sharing the cell), the gathered "appearances" of
@@ -418,6 +449,9 @@ std::shared_ptr<FdTables> build_local_solvers(const tpss_layout &L, const tpss_o
     T->rcp64.upload(r64.data(), r64.size());
     T->rcp32.upload(r32.data(), r32.size());
     T->rcp_E = -1;  // one table per patch
+    // the integer smoother reads these reciprocals, not the eigenvalue sums
+    T->fix_ok = std::all_of(T->S_host.begin(), T->S_host.end(), [](double v) { return std::fabs(v) < 1e30; }) &&
+                std::all_of(r64.begin(), r64.end(), [](double v) { return v > 1e-60 && v < 1e60; });
     T->learned_fallbacks = kept;
     T->setup_seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     return T;
@@ -664,6 +698,11 @@ void apply_color(tpss_precond *p, int color, double *dst, const double *src, cud
     a.entry_stride = (2 * L.n + 1) * p->tables->npad64;
     a.fd_eo = eo ? (const void *)p->tables->fd64_eo.ptr : nullptr;
     a.eo_stride = 4 * h * p->tables->hpad64 + p->tables->npad64;
+    a.fix = p->tables->fix64.ptr;
+    a.fix_eo = p->tables->fix64_eo.ptr;
+    a.fexp = p->tables->fexp.ptr;
+    a.fexp_eo = p->tables->fexp_eo.ptr;
+    a.fp64_only = !p->tables->fix_ok;
     ok = launch_fd_f64(L.dim, L.k, L.ncp, a, s);
   }
   if(!ok)
