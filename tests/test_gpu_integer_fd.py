@@ -88,3 +88,39 @@ def check_range_and_nan(tpss, oracle, cuda, dim, k, nc, **kw):
 @pytest.mark.parametrize("dim,k,nc", [(2, 3, (9, 7)), (3, 2, (5, 4, 6)), (3, 4, (4, 4, 3))])
 def test_color_kernel_range_and_nan(tpss, oracle, cuda, dim, k, nc):
     check_range_and_nan(tpss, oracle, cuda, dim, k, nc, kernel_variant=1)
+
+
+# vertices along x around the tile of 8 (4 for k >= 5 in 3D) and cells around 7 (3); one patch; line
+# counts below and above one CTA's 128; lines long enough to be cut into segments
+SWEEP = [(2, 1, (2, 2)), (2, 3, (8, 5)), (2, 3, (9, 4)), (2, 4, (3, 70)), (2, 7, (15, 3)), (2, 2, (40, 3)), (3, 1, (2, 2, 2)),
+         (3, 1, (16, 2, 9)), (3, 2, (7, 5, 4)), (3, 3, (4, 3, 21)), (3, 4, (9, 2, 3)), (3, 5, (5, 4, 2)), (3, 6, (2, 3, 2)),
+         (3, 7, (4, 2, 2))]
+
+
+@pytest.mark.parametrize("dim,k,nc", SWEEP)
+def test_direction_sweep(tpss, oracle, cuda, dim, k, nc):
+    """The direction-by-direction smoother (the default for FP64 additive vertex patches) against the
+    oracle on uniform cells, and on all against the per-color kernel, which reads the same tables;
+    unequal widths (with k = 7 too many entry combinations for tabulated reciprocals; their 1-D
+    eigenproblems are so ill-conditioned that either kernel differs from the oracle's own
+    eigensolver by up to 1.5e-11), permuted cells, RAS weights."""
+    nd = (k + 1) ** dim
+    src = philox(20 + k, int(np.prod(nc)) * nd)
+    om = 0.37
+    cells = np.random.Generator(np.random.Philox(5)).permutation(int(np.prod(nc))).astype(np.int64) * nd
+    for h, cs, ras in ((None, None, False), (widths(nc, k), None, True), (widths(nc, k + 1), cells, False)):
+        kw = dict(h=h, cells=cs, relaxation=om, use_ras_weights=ras)
+        got = apply(make(tpss, dim, k, nc, **kw), src, cuda)
+        if h is None:
+            ref = oracle.schwarz_vmult(dim, k, nc, src, omega=om)
+            assert rel_err(got, ref) <= 1e-12
+        assert rel_err(got, apply(make(tpss, dim, k, nc, kernel_variant=1, **kw), src, cuda)) <= 1e-12
+    p = make(tpss, dim, k, nc, relaxation=om)
+    ref = oracle.schwarz_vmult(dim, k, nc, src, omega=om)
+    for scale in (2.0 ** 290, 2.0 ** -290, 2.0 ** 320, 2.0 ** -320):
+        assert rel_err(apply(p, src * scale, cuda) / scale, ref) <= 1e-12, scale
+
+
+@pytest.mark.parametrize("dim,k,nc", [(2, 3, (9, 7)), (3, 2, (5, 4, 6)), (3, 4, (4, 4, 3))])
+def test_direction_sweep_range_and_nan(tpss, oracle, cuda, dim, k, nc):
+    check_range_and_nan(tpss, oracle, cuda, dim, k, nc)

@@ -132,8 +132,6 @@ __device__ __forceinline__ void row_dot(const int2 *__restrict__ row, const int 
                                         int64_t (&y)[P])
 {
   Acc M[P], S[P];
-#pragma unroll
-  for(int p = 0; p < P; ++p) M[p] = Acc(1u << 31);
   const int4 *row4 = reinterpret_cast<const int4 *>(row);
 #pragma unroll
   for(int j2 = 0; j2 < (H + 1) / 2; ++j2)
@@ -142,7 +140,8 @@ __device__ __forceinline__ void row_dot(const int2 *__restrict__ row, const int 
 #pragma unroll
     for(int p = 0; p < P; ++p)
     {
-      M[p].add(c.y, xl[p][2 * j2]);
+      if(j2 == 0) M[p].start(c.y, xl[p][0]);
+      else M[p].add(c.y, xl[p][2 * j2]);
       M[p].add(c.x, xh[p][2 * j2]);
       if(j2 == 0) S[p].start(c.y, xh[p][0]);
       else S[p].add(c.y, xh[p][2 * j2]);
@@ -159,8 +158,9 @@ __device__ __forceinline__ void row_dot(const int2 *__restrict__ row, const int 
       }
     }
   }
+  // rounded to the nearest unit from M's low word (which also keeps its last product one instruction)
 #pragma unroll
-  for(int p = 0; p < P; ++p) y[p] = S[p].value() + M[p].hi;
+  for(int p = 0; p < P; ++p) y[p] = S[p].value() + (M[p].hi + (int)(M[p].lo >> 31));
 }
 }  // namespace fx
 }  // namespace tpss

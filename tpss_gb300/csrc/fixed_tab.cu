@@ -53,20 +53,20 @@ __global__ void __launch_bounds__(64) fixed_table_kernel(const double *__restric
 
 void build_fixed_tables(FdTables &T)
 {
-  if(T.n_entries == 0) return;
+  static std::mutex mu;  // tables are shared by shallow copies
+  std::lock_guard<std::mutex> lock(mu);
+  if(T.n_entries == 0 || T.fix64) return;
   const int n = T.n, h = n / 2;
-  const int es = (2 * n + 1) * T.npad64, es_eo = 4 * h * T.hpad64 + T.npad64;
-  T.fix64.resize((size_t)T.n_entries * es);
-  T.fexp.resize(T.n_entries);
-  fixed_table_kernel<<<T.n_entries, 64>>>(T.fd64.ptr, n, T.npad64, es, T.fix64.ptr, T.fexp.ptr);
+  const size_t E = T.n_entries, es = (2 * n + 1) * T.npad64, es_eo = T.has_eo ? 4 * h * T.hpad64 + T.npad64 : 0;
+  T.fix_buf.resize(E * (es + es_eo + 2));
+  int2 *fix = T.fix_buf.ptr, *eo = fix + E * es, *fe = eo + E * es_eo;
+  fixed_table_kernel<<<T.n_entries, 64>>>(T.fd64.ptr, n, T.npad64, (int)es, fix, fe);
+  if(T.has_eo) fixed_table_kernel<<<T.n_entries, 64>>>(T.fd64_eo.ptr, 2 * h, T.hpad64, (int)es_eo, eo, fe + E);
   TPSS_CUDA(cudaGetLastError());
-  if(T.has_eo)
-  {
-    T.fix64_eo.resize((size_t)T.n_entries * es_eo);
-    T.fexp_eo.resize(T.n_entries);
-    fixed_table_kernel<<<T.n_entries, 64>>>(T.fd64_eo.ptr, 2 * h, T.hpad64, es_eo, T.fix64_eo.ptr, T.fexp_eo.ptr);
-    TPSS_CUDA(cudaGetLastError());
-  }
-  TPSS_CUDA(cudaDeviceSynchronize());
+  TPSS_CUDA(cudaStreamSynchronize(nullptr));  // the tables are read on any stream
+  T.fix64 = fix;
+  T.fix64_eo = eo;
+  T.fexp = fe;
+  T.fexp_eo = fe + E;
 }
 }  // namespace tpss

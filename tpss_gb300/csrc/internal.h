@@ -258,10 +258,13 @@ struct FdTables
   DeviceBuffer<double> fd64_eo;  // the same in FP64 (per-color kernel, FP64 smoother)
   DeviceBuffer<int32_t> sym;
   bool has_eo = false;           // some entry has the even/odd form
-  // FP64 smoother on the integer pipe (fd_fixed.cuh): the coefficients of fd64 and fd64_eo as 64-bit
-  // integers c 2^F in signed 32-bit limbs, same strides (the eigenvalue words unused), and per
-  // entry F of S^T and of S
-  DeviceBuffer<int2> fix64, fix64_eo, fexp, fexp_eo;
+  // FP64 smoother on the integer pipe (fd_fixed.cuh, sweep64.cuh), built for FP64 preconditioners: the
+  // coefficients of fd64 and fd64_eo as 64-bit integers c 2^F in signed 32-bit limbs, same strides
+  // (the eigenvalue words unused), and per entry F of S^T and of S; all in one buffer
+  DeviceBuffer<int2> fix_buf;
+  const int2 *fix64 = nullptr, *fix64_eo = nullptr, *fexp = nullptr, *fexp_eo = nullptr;
+  // eigenvalue per direction and vertex mode ((vertex - 1) n + i), where rcp64 is empty
+  DeviceBuffer<double> lam_modes[3];
   bool fix_ok = false;           // finite tables and positive eigenvalue sums: the integers apply
   // eigenvalues of every entry in the order the kernels read them (the even/odd order for
   // mirror-symmetric entries), n_entries x n, host
@@ -344,6 +347,7 @@ struct tpss_precond
   tpss_precond_desc desc{};
   tpss::DeviceBuffer<double> residual;  // multiplicative scratch
   tpss::DeviceBuffer<int> flag;         // finiteness check
+  tpss::DeviceBuffer<double> sweep[3];  // direction-by-direction smoother: line arrays (sweep64.cuh)
   tpss::DeviceBuffer<float> halo;       // streamed kernel: partial sums of shared cells
   tpss::DeviceBuffer<int64_t> fix_rec[8];  // streamed kernel: shared-cell list per variant
   int64_t fix_n[8] = {-1, -1, -1, -1, -1, -1, -1, -1};
@@ -403,7 +407,7 @@ bool mapped_apply_mf(const tpss_operator &op, double *dst, const double *src, cu
 // its FP32 arithmetic (FP32 copies of the cell blocks, face geometry and source; FP64 result)
 bool mapped_apply_mf_f32(tpss_operator &op, double *dst, const double *src, cudaStream_t s,
                          const double *rhs = nullptr);
-// integer forms of the FP64 tables (fixed_tab.cu)
+// integer forms of the FP64 tables (fixed_tab.cu); does nothing when they are there
 void build_fixed_tables(FdTables &T);
 // FD setup helpers (precond.cu, eigen.cu)
 void gen_eig_batched(int n, int n_problems, const std::vector<double> &Ms,
@@ -500,6 +504,21 @@ bool launch_stream3d_host_k5(const tpss_layout &L, const StreamLaunch &l, HostPi
                              const double *h_src, cudaStream_t s);
 int stream_variant_count(const tpss_layout &L);
 bool launch_stream3d(const tpss_layout &L, const StreamLaunch &l, cudaStream_t s);
+
+// direction-by-direction FP64 smoother of additive vertex patches on a Cartesian level (sweep64.cu)
+struct SweepLaunch
+{
+  const tpss_layout *layout;
+  const FdTables *tables;
+  const double *src;
+  double *dst;
+  double *a, *b, *c;  // line arrays
+  double omega;
+  int ras;
+};
+bool launch_sweep_0(const SweepLaunch &l, cudaStream_t s);
+bool launch_sweep_1(const SweepLaunch &l, cudaStream_t s);
+bool launch_sweep_2(const SweepLaunch &l, cudaStream_t s);
 
 // upload the layout's index tables (layout.cu)
 void layout_to_device(const tpss_layout &L);

@@ -9,6 +9,7 @@
 // level operator between colors in the color sequence of get_color_sequence
 // (schwarz_preconditioner.h:532-567, templates:691-732).
 #include <algorithm>
+#include <array>
 #include <chrono>
 #include <cmath>
 #include <cstring>
@@ -297,7 +298,20 @@ std::shared_ptr<FdTables> build_tables(const tpss_layout &L, Penalty ip, bool ra
   T->fd32.upload(t32.data(), t32.size());
   build_even_odd(L, *T, Ms, As, keyed);
   if(keyed) build_reciprocals(L, *T);
-  build_fixed_tables(*T);
+  if(keyed && T->rcp_E == 0)
+    for(int d = 0; d < L.dim; ++d)
+    {
+      // eigenvalues per vertex and mode, in the kernels' order (empty unless the key depends on the
+      // vertex index alone)
+      if(L.vertex_fd[d].empty()) continue;
+      std::vector<double> lam;
+      for(int v = 1; v < L.nc[d]; ++v)
+      {
+        const double *l = &T->lam_kernel[(size_t)L.vertex_fd[d][v] * n];
+        lam.insert(lam.end(), l, l + n);
+      }
+      T->lam_modes[d].upload(lam.data(), lam.size());
+    }
   T->fix_ok = fixed_applies(L, *T, keyed);
   if(ras)
   {
@@ -698,10 +712,10 @@ void apply_color(tpss_precond *p, int color, double *dst, const double *src, cud
     a.entry_stride = (2 * L.n + 1) * p->tables->npad64;
     a.fd_eo = eo ? (const void *)p->tables->fd64_eo.ptr : nullptr;
     a.eo_stride = 4 * h * p->tables->hpad64 + p->tables->npad64;
-    a.fix = p->tables->fix64.ptr;
-    a.fix_eo = p->tables->fix64_eo.ptr;
-    a.fexp = p->tables->fexp.ptr;
-    a.fexp_eo = p->tables->fexp_eo.ptr;
+    a.fix = p->tables->fix64;
+    a.fix_eo = p->tables->fix64_eo;
+    a.fexp = p->tables->fexp;
+    a.fexp_eo = p->tables->fexp_eo;
     a.fp64_only = !p->tables->fix_ok;
     ok = launch_fd_f64(L.dim, L.k, L.ncp, a, s);
   }
@@ -764,6 +778,71 @@ bool use_stream(const tpss_precond *p)
   return ok;
 }
 
+namespace
+{
+// the direction-by-direction FP64 smoother applies: additive vertex patches of a Cartesian level
+// with keyed fast-diagonalization tables and at least one patch
+bool sweep_eligible(const tpss_precond *p)
+{
+  const tpss_layout &L = *p->tables->layout;
+  if(p->desc.precision != TPSS_FP64 || p->desc.kernel_variant != TPSS_KERNEL_AUTO) return false;
+  if(L.smoother_variant != TPSS_ADDITIVE || L.patch_variant != TPSS_PATCH_VERTEX || L.per_patch_fd) return false;
+  if(p->tables->dense || p->tables->own_fd.n || p->tables->rcp_E < 0 || p->desc.use_ras_boolean_weights) return false;
+  return L.P > 0 && !L.vertex_fd[0].empty();
+}
+
+// line arrays of the sweep: values per array (T1 / U1, T2, U2; 2D: T1, U1)
+std::array<size_t, 3> sweep_sizes(const tpss_layout &L)
+{
+  const size_t mx = (size_t)(L.nc[0] - 1) * L.n, gy = (size_t)L.nc[1] * L.np;
+  if(L.dim == 2) return {mx * gy, mx * gy, 0};
+  const size_t my = (size_t)(L.nc[1] - 1) * L.n, gz = (size_t)L.nc[2] * L.np;
+  return {mx * gy * gz, mx * my * gz, mx * my * gz};
+}
+
+// Holds the line arrays, or gets them if it may: not inside a stream capture, and not when the device
+// has no room for them (the per-color kernel then does without).
+bool sweep_scratch(tpss_precond *p, cudaStream_t s)
+{
+  const auto n = sweep_sizes(*p->tables->layout);
+  bool have = true;
+  for(int i = 0; i < 3; ++i) have = have && p->sweep[i].n >= n[i];
+  if(have) return true;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  cudaStreamIsCapturing(s, &cs);
+  if(cs != cudaStreamCaptureStatusNone) return false;
+  try
+  {
+    for(int i = 0; i < 3; ++i)
+      if(p->sweep[i].n < n[i]) p->sweep[i].resize(n[i]);
+  }
+  catch(const Error &e)
+  {
+    cudaGetLastError();
+    for(auto &b : p->sweep) b.release();
+    return false;
+  }
+  return true;
+}
+
+void launch_sweep(tpss_precond *p, double *dst, const double *src, cudaStream_t s)
+{
+  SweepLaunch l;
+  l.layout = p->tables->layout;
+  l.tables = p->tables.get();
+  l.src = src;
+  l.dst = dst;
+  l.a = p->sweep[0].ptr;
+  l.b = p->sweep[1].ptr;
+  l.c = p->sweep[2].ptr;
+  l.omega = p->desc.relaxation;
+  l.ras = p->desc.use_ras_weights != 0;
+  const int part = l.layout->k % 3;
+  const bool ok = part == 0 ? launch_sweep_0(l, s) : part == 1 ? launch_sweep_1(l, s) : launch_sweep_2(l, s);
+  if(!ok) fail(TPSS_ERR_NOT_IMPLEMENTED, "FP64 sweep: unsupported degree");
+}
+}  // namespace
+
 StreamLaunch stream_launch(tpss_precond *p, double *dst, const double *src)
 {
   const tpss_layout &L = *p->tables->layout;
@@ -813,12 +892,15 @@ void precond_vmult(tpss_precond *p, double *dst, const double *src, cudaStream_t
   TPSS_REQUIRE(dst && src, "null vector");
   TPSS_REQUIRE(dst != src, "dst and src must not alias");
   ScopedTimer step(p, 4, s);
-  if(!(L.smoother_variant == TPSS_ADDITIVE && use_stream(p)))
+  const bool sweep = sweep_eligible(p) && sweep_scratch(p, s);
+  if(!sweep && !(L.smoother_variant == TPSS_ADDITIVE && use_stream(p)))
     TPSS_CUDA(cudaMemsetAsync(dst, 0, sizeof(double) * L.n_dofs, s));
   if(L.smoother_variant == TPSS_ADDITIVE)
   {
     ScopedTimer t(p, 1, s);
-    if(use_stream(p))
+    if(sweep)
+      launch_sweep(p, dst, src, s);  // writes every cell of dst
+    else if(use_stream(p))
     {
       // one pass over all patches; every cell of dst is written, no zeroing needed
       const StreamLaunch l = stream_launch(p, dst, src);
@@ -898,6 +980,8 @@ extern "C" int tpss_precond_create(const tpss_layout *layout, tpss_operator *op,
     p->color_variant = desc->stream_variant;  // variants the kernel does not offer fall back to 0
     p->tables = build_local_solvers(*layout, op, *desc);
     if(desc->use_ras_boolean_weights) build_keep_tables(*layout, *p->tables);
+    if(desc->precision == TPSS_FP64) build_fixed_tables(*p->tables);
+    if(sweep_eligible(p.get())) sweep_scratch(p.get(), nullptr);
     p->timers.resize(5);
     for(int i = 0; i < 5; ++i) p->timers[i].name = kTimerNames[i];
     p->timers[2].time = p->tables->setup_seconds;
@@ -930,6 +1014,7 @@ extern "C" int tpss_precond_create_shallow(const tpss_precond *other, const tpss
       fail(TPSS_ERR_INVALID_ARGUMENT, "shallow copy cannot add RAS weights");
     validate_ras_boolean(*p->tables->layout, *desc);
     if(desc->use_ras_boolean_weights) build_keep_tables(*p->tables->layout, *p->tables);
+    if(desc->precision == TPSS_FP64) build_fixed_tables(*p->tables);
     p->timers = other->timers;
     *out = p.release();
   });
@@ -1072,7 +1157,7 @@ extern "C" int tpss_precond_autotune(tpss_precond *p, double *dst, const double 
     // (dense local inverses have a single kernel)
     const bool streamed = use_stream(p);
     const int nv = streamed ? stream_variant_count(L)
-                   : p->tables->dense ? 1
+                   : p->tables->dense || (sweep_eligible(p) && sweep_scratch(p, s)) ? 1
                                       : fd_variants(p->desc.precision == TPSS_FP32, L.dim, L.k, L.ncp);
     int &variant = streamed ? p->stream_variant : p->color_variant;
     if(n_variants) *n_variants = nv;
