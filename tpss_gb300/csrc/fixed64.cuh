@@ -100,6 +100,26 @@ __device__ __forceinline__ int64_t from_double(double v, int emax)
   return (a ^ s) - s;
 }
 
+// y 2^ex as a double (ex keeps the result in the normal range). The conversion instruction is an FP64
+// one (64 clocks of a warp's FP64 pipe); to_double_alu does it in about 20 integer operations (40
+// clocks of another pipe), rounding half up. Kernels split their results between the two.
+__device__ __forceinline__ double to_double(int64_t y, int ex)
+{
+  const double d = __ll2double_rn(y);
+  const int hi = y == 0 ? 0 : __double2hiint(d) + ex * (1 << 20);
+  return __hiloint2double(hi, __double2loint(d));
+}
+
+__device__ __forceinline__ double to_double_alu(int64_t y, int ex)
+{
+  const int64_t s = y >> 63;
+  const uint64_t a = (uint64_t)((y ^ s) - s);
+  const int up = __clzll((long long)a) - 1;  // leading bit to bit 62
+  const uint64_t m = ((a << (up & 63)) + 0x200) >> 10;  // leading bit at 52, or 53 after a carry
+  const int hi = (int)(m >> 32) + ((ex + 1084 - up) << 20);
+  return a == 0 ? 0.0 : __hiloint2double(hi | (int)((unsigned)(s >> 32) & 0x80000000u), (int)m);
+}
+
 // 2^e as a double, e in [-1022, 1023]
 __device__ __forceinline__ double pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }
 
@@ -126,10 +146,11 @@ __device__ __forceinline__ int64_t mul_m61(int64_t x, int mh, int ml)
 }
 
 // ---- coefficient rows: int2 (x: low limb, y: high limb), read as pairs
-// y[p] = sum_j c_j x_j / 2^64 of one row of H coefficients for P vectors x in limbs
-template<int H, int P>
-__device__ __forceinline__ void row_dot(const int2 *__restrict__ row, const int (&xh)[P][H], const int (&xl)[P][H],
-                                        int64_t (&y)[P])
+// y[p] = sum_j c_j x_j / 2^64 of one row of H coefficients for P vectors x in limbs (the first H of L
+// values each)
+template<int H, int L, int P>
+__device__ __forceinline__ void row_dot_n(const int2 *__restrict__ row, const int (&xh)[P][L], const int (&xl)[P][L],
+                                          int64_t (&y)[P])
 {
   Acc M[P], S[P];
   const int4 *row4 = reinterpret_cast<const int4 *>(row);
@@ -161,6 +182,13 @@ __device__ __forceinline__ void row_dot(const int2 *__restrict__ row, const int 
   // rounded to the nearest unit from M's low word (which also keeps its last product one instruction)
 #pragma unroll
   for(int p = 0; p < P; ++p) y[p] = S[p].value() + (M[p].hi + (int)(M[p].lo >> 31));
+}
+
+template<int H, int P>
+__device__ __forceinline__ void row_dot(const int2 *__restrict__ row, const int (&xh)[P][H], const int (&xl)[P][H],
+                                        int64_t (&y)[P])
+{
+  row_dot_n<H, H, P>(row, xh, xl, y);
 }
 }  // namespace fx
 }  // namespace tpss

@@ -67,6 +67,46 @@ int guarded(F &&f)
   }
 }
 
+// Orders uses of a handle's scratch: a call waits for the previous one's work, also when that went to
+// another stream or came from another thread. A stream capture cannot wait for work outside it; a
+// captured call uses the scratch as it is (as the handle's contract has it, one stream at a time).
+struct ScratchOrder
+{
+  std::mutex m;
+  cudaEvent_t ev = nullptr;
+  ScratchOrder() = default;
+  ScratchOrder(const ScratchOrder &) = delete;
+  ~ScratchOrder()
+  {
+    if(ev) cudaEventDestroy(ev);
+  }
+};
+
+class ScratchUse
+{
+  ScratchOrder &o;
+  std::lock_guard<std::mutex> lock;
+  cudaStream_t s;
+  bool capturing = false;
+
+public:
+  ScratchUse(ScratchOrder &order, cudaStream_t stream) : o(order), lock(order.m), s(stream)
+  {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    TPSS_CUDA(cudaStreamIsCapturing(s, &cs));
+    capturing = cs != cudaStreamCaptureStatusNone;
+    if(capturing) return;
+    if(o.ev) TPSS_CUDA(cudaStreamWaitEvent(s, o.ev, 0));
+    else TPSS_CUDA(cudaEventCreateWithFlags(&o.ev, cudaEventDisableTiming));
+  }
+  ScratchUse(const ScratchUse &) = delete;
+  ~ScratchUse()
+  {
+    if(!capturing) cudaEventRecord(o.ev, s);
+  }
+  bool may_allocate() const { return !capturing; }
+};
+
 // device buffer with RAII
 template<typename T>
 struct DeviceBuffer
@@ -223,6 +263,19 @@ struct MappedOperator
 };
 }  // namespace tpss
 
+namespace tpss
+{
+// line-by-line FP64 operator (sipg_lines.cu): tables of all directions in one buffer, and the
+// intermediate vectors (4 per level in 3D, 2 in 2D)
+struct OpLines
+{
+  DeviceBuffer<int64_t> tables;
+  size_t off_tab[3] = {}, off_tab64[3] = {}, off_sig[3] = {}, off_exps[3] = {}, off_width[3] = {};
+  DeviceBuffer<double> buf;
+  ScratchOrder order;
+};
+}  // namespace tpss
+
 struct tpss_operator
 {
   const tpss_layout *layout = nullptr;
@@ -232,6 +285,7 @@ struct tpss_operator
   tpss::DeviceBuffer<double> d_fac[3];  // operator_factors_1d per direction
   tpss::DeviceBuffer<float> d_fac32[3];  // the same in FP32 (single-precision level operator)
   tpss::DeviceBuffer<float> x32;         // FP32 copy of the source (single-precision operator)
+  tpss::OpLines lines;                   // FP64, Cartesian levels
   bool sparse_faces = false;             // face couplings with unit value vectors (operator.cu)
   int nblk_cells[3] = {0, 0, 0};
   std::unique_ptr<tpss::MappedOperator> mapped;  // set on distorted levels
@@ -348,6 +402,7 @@ struct tpss_precond
   tpss::DeviceBuffer<double> residual;  // multiplicative scratch
   tpss::DeviceBuffer<int> flag;         // finiteness check
   tpss::DeviceBuffer<double> sweep[3];  // direction-by-direction smoother: line arrays (sweep64.cuh)
+  tpss::ScratchOrder sweep_order;
   tpss::DeviceBuffer<float> halo;       // streamed kernel: partial sums of shared cells
   tpss::DeviceBuffer<int64_t> fix_rec[8];  // streamed kernel: shared-cell list per variant
   int64_t fix_n[8] = {-1, -1, -1, -1, -1, -1, -1, -1};
@@ -446,6 +501,10 @@ void extract_local_matrices(const tpss_layout &L, const tpss_operator &op, int64
 // dst = A src, or with rhs the residual dst = rhs - A src
 void operator_apply(tpss_operator *op, double *dst, const double *src, cudaStream_t s,
                     const double *rhs = nullptr);
+// line-by-line form of the FP64 product on a Cartesian level; false without tables or room for its
+// intermediate vectors (also while a stream is captured before the first product)
+void build_op_lines(tpss_operator &op, const tpss_layout &L, Penalty pen);
+bool op_lines_apply(tpss_operator &op, double *dst, const double *src, cudaStream_t s, const double *rhs);
 // the same operator in FP32 arithmetic (FP64 vectors; the source is converted once into a
 // scratch copy): for the residuals inside a single-precision V-cycle (distorted levels: FP32
 // copy of the block-sparse matrix)

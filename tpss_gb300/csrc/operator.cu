@@ -642,6 +642,7 @@ void operator_apply(tpss_operator *op, double *dst, const double *src, cudaStrea
     mapped_apply(*op, dst, src, s, rhs);
     return;
   }
+  if(op_lines_apply(*op, dst, src, s, rhs)) return;
   const OpArgs<double> a = op_args<double>(*op, src, dst, rhs);
   TPSS_DISPATCH_NP(L.dim, L.np, launch_sipg, a, s);
 }
@@ -776,6 +777,7 @@ extern "C" int tpss_operator_create_penalty(const tpss_layout *layout, double ip
       op->d_fac32[d].upload(fac32.data(), fac32.size());
       op->nblk_cells[d] = layout->nc[d];
     }
+    build_op_lines(*op, *layout, pen);
     *out = op.release();
   });
 }

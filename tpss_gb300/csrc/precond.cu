@@ -13,6 +13,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstring>
+#include <optional>
 
 #include "internal.h"
 
@@ -802,15 +803,13 @@ std::array<size_t, 3> sweep_sizes(const tpss_layout &L)
 
 // Holds the line arrays, or gets them if it may: not inside a stream capture, and not when the device
 // has no room for them (the per-color kernel then does without).
-bool sweep_scratch(tpss_precond *p, cudaStream_t s)
+bool sweep_scratch(tpss_precond *p, bool may_allocate)
 {
   const auto n = sweep_sizes(*p->tables->layout);
   bool have = true;
   for(int i = 0; i < 3; ++i) have = have && p->sweep[i].n >= n[i];
   if(have) return true;
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  cudaStreamIsCapturing(s, &cs);
-  if(cs != cudaStreamCaptureStatusNone) return false;
+  if(!may_allocate) return false;
   try
   {
     for(int i = 0; i < 3; ++i)
@@ -892,14 +891,20 @@ void precond_vmult(tpss_precond *p, double *dst, const double *src, cudaStream_t
   TPSS_REQUIRE(dst && src, "null vector");
   TPSS_REQUIRE(dst != src, "dst and src must not alias");
   ScopedTimer step(p, 4, s);
-  const bool sweep = sweep_eligible(p) && sweep_scratch(p, s);
+  std::optional<ScratchUse> use;
+  if(sweep_eligible(p)) use.emplace(p->sweep_order, s);
+  const bool sweep = use && sweep_scratch(p, use->may_allocate());
+  if(!sweep) use.reset();
   if(!sweep && !(L.smoother_variant == TPSS_ADDITIVE && use_stream(p)))
     TPSS_CUDA(cudaMemsetAsync(dst, 0, sizeof(double) * L.n_dofs, s));
   if(L.smoother_variant == TPSS_ADDITIVE)
   {
     ScopedTimer t(p, 1, s);
     if(sweep)
+    {
       launch_sweep(p, dst, src, s);  // writes every cell of dst
+      use.reset();
+    }
     else if(use_stream(p))
     {
       // one pass over all patches; every cell of dst is written, no zeroing needed
@@ -981,7 +986,7 @@ extern "C" int tpss_precond_create(const tpss_layout *layout, tpss_operator *op,
     p->tables = build_local_solvers(*layout, op, *desc);
     if(desc->use_ras_boolean_weights) build_keep_tables(*layout, *p->tables);
     if(desc->precision == TPSS_FP64) build_fixed_tables(*p->tables);
-    if(sweep_eligible(p.get())) sweep_scratch(p.get(), nullptr);
+    if(sweep_eligible(p.get())) sweep_scratch(p.get(), true);
     p->timers.resize(5);
     for(int i = 0; i < 5; ++i) p->timers[i].name = kTimerNames[i];
     p->timers[2].time = p->tables->setup_seconds;
@@ -1157,7 +1162,7 @@ extern "C" int tpss_precond_autotune(tpss_precond *p, double *dst, const double 
     // (dense local inverses have a single kernel)
     const bool streamed = use_stream(p);
     const int nv = streamed ? stream_variant_count(L)
-                   : p->tables->dense || (sweep_eligible(p) && sweep_scratch(p, s)) ? 1
+                   : p->tables->dense || (sweep_eligible(p) && sweep_scratch(p, true)) ? 1
                                       : fd_variants(p->desc.precision == TPSS_FP32, L.dim, L.k, L.ncp);
     int &variant = streamed ? p->stream_variant : p->color_variant;
     if(n_variants) *n_variants = nv;

@@ -1,0 +1,340 @@
+// sipg_lines.cu -- tables and launches of the line-by-line FP64 SIPG operator (sipg_lines.cuh).
+#include <cmath>
+#include <cstring>
+#include <map>
+#include <type_traits>
+
+#include "internal.h"
+#include "sipg_lines.cuh"
+
+namespace tpss
+{
+using namespace lines;
+
+namespace
+{
+// 1-D reference element in extended precision: the integers of the tables hold 62 bits, and the rounding
+// of the FP64 basis (some 1e-15 of an entry for high degrees) would be the operator's largest error.
+// mass and stiffness on [0, 1], derivatives at the upper end (those at the lower end mirror them)
+template<int N>
+struct Element
+{
+  long double mass[N][N], stiff[N][N], g[N];
+};
+
+template<int N>
+Element<N> make_element(const Shape1D &s)
+{
+  using R = long double;
+  // P_m and its derivative at z in (-1, 1)
+  auto legendre = [](int m, R z, R &p, R &dp) {
+    R p0 = 1, p1 = z;
+    for(int j = 2; j <= m; ++j)
+    {
+      const R p2 = ((2 * j - 1) * z * p1 - (j - 1) * p0) / j;
+      p0 = p1;
+      p1 = p2;
+    }
+    p = p1;
+    dp = m * (z * p1 - p0) / (z * z - 1);
+  };
+  // the FP64 points, one Newton step each (quadratic: twice as many digits), by symmetry in pairs
+  R x[N], qx[N], qw[N];
+  x[0] = 0;
+  x[N - 1] = 1;
+  for(int i = 0; i < N; ++i)
+  {
+    R z = 2 * (R)s.qx[i] - 1, p, dp;
+    legendre(N, z, p, dp);
+    z -= p / dp;
+    legendre(N, z, p, dp);
+    qx[i] = (1 + z) / 2;
+    qw[i] = 1 / ((1 - z * z) * dp * dp);
+    if(i == 0 || i == N - 1) continue;
+    z = 2 * (R)s.nodes[i] - 1;
+    legendre(N - 1, z, p, dp);
+    z -= dp * (1 - z * z) / (2 * z * dp - (R)(N - 1) * N * p);
+    x[i] = (1 + z) / 2;
+  }
+  auto lagrange = [&](R at, R(&v)[N], R(&d)[N]) {
+    for(int i = 0; i < N; ++i)
+    {
+      v[i] = 1;
+      d[i] = 0;
+      for(int j = 0; j < N; ++j)
+      {
+        if(j == i) continue;
+        d[i] = (d[i] * (at - x[j]) + v[i]) / (x[i] - x[j]);
+        v[i] *= (at - x[j]) / (x[i] - x[j]);
+      }
+    }
+  };
+  Element<N> e{};
+  R v[N], d[N];
+  for(int q = 0; q < N; ++q)
+  {
+    lagrange(qx[q], v, d);
+    for(int i = 0; i < N; ++i)
+      for(int j = 0; j < N; ++j)
+      {
+        e.mass[i][j] += v[i] * v[j] * qw[q];
+        e.stiff[i][j] += d[i] * d[j] * qw[q];
+      }
+  }
+  lagrange(1, v, e.g);
+  return e;
+}
+
+// Table of one cell width h (layout OpTab<N>)
+template<int N>
+void fill_table(const Element<N> &s, double h, long double sigma, std::vector<long double> &t)
+{
+  using T = OpTab<N>;
+  constexpr int H = T::H, HE = T::HE;
+  t.assign(T::SIZE, 0.0L);
+  // own block: stiffness and the cell's own terms of two interior faces with penalty sigma (the basis is
+  // 1 at its own face node and 0 at the others); trace towards the upper neighbour
+  long double M[N][N], C[N][N], b[N], g[N];
+  for(int j = 0; j < N; ++j)
+  {
+    g[j] = s.g[j] / h;
+    b[j] = 0.5L * g[j] - (j == N - 1 ? sigma : 0.0L);
+  }
+  for(int i = 0; i < N; ++i)
+    for(int j = 0; j < N; ++j)
+    {
+      M[i][j] = s.mass[i][j] * h;
+      C[i][j] = s.stiff[i][j] / h;
+      // outward derivatives: g at the upper face, mirrored at the lower one
+      const long double v1 = i == N - 1, u1 = j == N - 1, v0 = i == 0, u0 = j == 0;
+      C[i][j] += sigma * (v1 * u1 + v0 * u0) - 0.5L * (g[j] * v1 + g[i] * u1 + g[N - 1 - j] * v0 + g[N - 1 - i] * u0);
+    }
+  auto even = [&](auto at, int i, int j) { return 2 * j == N - 1 ? at(i, j) : 0.5L * (at(i, j) + at(i, N - 1 - j)); };
+  auto odd = [&](auto at, int i, int j) { return 0.5L * (at(i, j) - at(i, N - 1 - j)); };
+  auto m = [&](int i, int j) { return M[i][j]; };
+  auto c = [&](int i, int j) { return C[i][j]; };
+  auto tr = [&](int, int j) { return b[j]; };
+  for(int i = 0; i < HE; ++i)
+  {
+    for(int j = 0; j < HE; ++j)
+    {
+      t[T::ME + i * T::LME + j] = even(m, i, j);
+      t[T::CE + i * T::LCE + j] = even(c, i, j);
+    }
+    t[T::CE + i * T::LCE + HE] = 0.25L * (g[i] + g[N - 1 - i]);
+    if(i >= H) continue;
+    for(int j = 0; j < H; ++j)
+    {
+      t[T::MO + i * T::LMO + j] = odd(m, i, j);
+      t[T::CO + i * T::LCO + j] = odd(c, i, j);
+    }
+    t[T::CO + i * T::LCO + H] = 0.25L * (g[i] - g[N - 1 - i]);
+  }
+  for(int j = 0; j < HE; ++j) t[T::TE + j] = even(tr, 0, j);
+  for(int j = 0; j < H; ++j) t[T::TO + j] = odd(tr, 0, j);
+}
+
+// F with sum_j |c_j| 2^F <= 2^62 in every row of [b, e) with row length len (rows of two lengths)
+int scale_of(const std::vector<long double> &t, int b, int rows, int len, int b2, int rows2, int len2)
+{
+  double mx = 0.0;
+  for(int i = 0; i < rows + rows2; ++i)
+  {
+    double s = 0.0;
+    for(int j = 0; j < (i < rows ? len : len2); ++j)
+      s += (double)std::fabs(t[i < rows ? b + i * len + j : b2 + (i - rows) * len2 + j]);
+    mx = std::max(mx, s * (1.0 + 1e-14));
+  }
+  int e = 0;
+  std::frexp(mx, &e);
+  return 62 - e;
+}
+
+template<int N>
+void build(tpss_operator &op, const tpss_layout &L, Penalty pen)
+{
+  using T = OpTab<N>;
+  const Element<N> s = make_element<N>(make_shape_1d(L.k));
+  const double gamma = double(L.k) * (L.k + 1);
+  OpLines &O = op.lines;
+  // per direction: [integer tables][FP64 tables][sigma: 3 per cell][exponents: 3 per width][width per cell]
+  std::vector<int64_t> buf;
+  for(int d = 0; d < L.dim; ++d)
+  {
+    const int n = L.nc[d];
+    const double *h = L.h[d].data();
+    std::map<double, int> id;
+    std::vector<int32_t> width(n + n % 2, 0);
+    std::vector<double> t64;
+    std::vector<int> exps;
+    std::vector<int64_t> ti;
+    for(int c = 0; c < n; ++c)
+    {
+      auto it = id.find(h[c]);
+      if(it == id.end())
+      {
+        it = id.emplace(h[c], (int)id.size()).first;
+        std::vector<long double> t;
+        fill_table<N>(s, h[c], (long double)pen.in * gamma / h[c], t);
+        const int F[3] = {scale_of(t, T::ME, T::HE, T::LME, T::MO, T::H, T::LMO),
+                          scale_of(t, T::CE, T::HE, T::LCE, T::CO, T::H, T::LCO),
+                          scale_of(t, T::TE, 1, T::LME, T::TO, 1, T::LMO)};
+        for(int i = 0; i < T::SIZE; ++i)
+        {
+          const int f = i < T::CE ? F[0] : i < T::TE ? F[1] : F[2];
+          const int64_t v = std::llrint(std::ldexp(t[i], f));
+          const int32_t lo = (int32_t)(uint32_t)(uint64_t)v;
+          const int32_t hi = (int32_t)((v - lo) >> 32);
+          ti.push_back((int64_t)((uint64_t)(uint32_t)hi << 32 | (uint32_t)lo));
+        }
+        t64.insert(t64.end(), t.begin(), t.end());
+        exps.insert(exps.end(), F, F + 3);
+      }
+      width[c] = it->second;
+    }
+    std::vector<double> sig(3 * (size_t)n);
+    for(int c = 0; c < n; ++c)
+    {
+      sig[3 * c] = c == 0 ? pen.bd * 2.0 * gamma / h[c] : pen.in * 0.5 * gamma * (1.0 / h[c - 1] + 1.0 / h[c]);
+      sig[3 * c + 1] = c == n - 1 ? pen.bd * 2.0 * gamma / h[c] : pen.in * 0.5 * gamma * (1.0 / h[c] + 1.0 / h[c + 1]);
+      sig[3 * c + 2] = pen.in * gamma / h[c];
+      if(c == 0 || c == n - 1 || h[c - 1] != h[c] || h[c + 1] != h[c]) width[c] |= kSpecial;
+    }
+    if(exps.size() % 2) exps.push_back(0);
+    auto put = [&](const void *p, size_t words) {
+      const size_t at = buf.size();
+      buf.resize(at + words);
+      std::memcpy(buf.data() + at, p, words * 8);
+      return at;
+    };
+    if(buf.size() % 2) buf.push_back(0);  // table rows are read as 16-byte pairs
+    O.off_tab[d] = put(ti.data(), ti.size());
+    O.off_tab64[d] = put(t64.data(), t64.size());
+    O.off_sig[d] = put(sig.data(), sig.size());
+    O.off_exps[d] = put(exps.data(), exps.size() / 2);
+    O.off_width[d] = put(width.data(), width.size() / 2);
+  }
+  O.tables.upload(buf.data(), buf.size());
+}
+
+template<int DIM, int N>
+void run(const tpss_operator &op, double *buf, double *dst, const double *src, cudaStream_t s, const double *rhs)
+{
+  const tpss_layout &L = *op.layout;
+  const OpLines &O = op.lines;
+  const int64_t nd = L.n_dofs, gx = (int64_t)L.nc[0] * N, gy = (int64_t)L.nc[1] * N;
+  auto args = [&](int d) {
+    OpLineArgs a{};
+    const int64_t *b = O.tables.ptr;
+    a.tab = reinterpret_cast<const int2 *>(b + O.off_tab[d]);
+    a.tab64 = reinterpret_cast<const double *>(b + O.off_tab64[d]);
+    a.sig = reinterpret_cast<const double *>(b + O.off_sig[d]);
+    a.exps = reinterpret_cast<const int *>(b + O.off_exps[d]);
+    a.width = reinterpret_cast<const int32_t *>(b + O.off_width[d]);
+    a.cell_start = L.lexicographic ? nullptr : L.d_cell_start.ptr;
+    for(int e = 0; e < 3; ++e) a.nc[e] = L.nc[e];
+    return a;
+  };
+  {
+    using C = OpXCfg<DIM, N>;
+    OpLineArgs a = args(0);
+    a.q = src;
+    a.r = buf;
+    a.m = buf + nd;
+    if constexpr(C::smem() > 48 * 1024)  // per device; a cheap host call
+      TPSS_CUDA(cudaFuncSetAttribute(op_x_kernel<DIM, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem()));
+    const int ng = L.nc[1] * (DIM == 3 ? L.nc[2] : 1);
+    const dim3 grid((ng + C::XG - 1) / C::XG, (L.nc[0] + C::XC - 1) / C::XC);
+    op_x_kernel<DIM, N><<<grid, C::THREADS, C::smem(), s>>>(a);
+    TPSS_CUDA(cudaGetLastError());
+  }
+  auto line_launch = [&](auto mode, OpLineArgs a, int d) {
+    // segments as for the smoother's lines (sweep64.cu): enough threads to fill the chip
+    const int len = L.nc[d];
+    int64_t segs = ((int64_t)num_sms() * 2048 + a.ncol - 1) / a.ncol;
+    segs = std::min<int64_t>(std::max<int64_t>(segs, 1), len);
+    a.seg = (int)((len + segs - 1) / segs);
+    const dim3 grid((unsigned)((a.ncol + kOpThreads - 1) / kOpThreads), (unsigned)((len + a.seg - 1) / a.seg));
+    op_line_kernel<DIM, N, decltype(mode)::value><<<grid, kOpThreads, 0, s>>>(a);
+    TPSS_CUDA(cudaGetLastError());
+  };
+  if constexpr(DIM == 3)
+  {
+    OpLineArgs a = args(1);
+    a.p = buf;
+    a.q = buf + nd;
+    a.r = buf + 2 * nd;
+    a.m = buf + 3 * nd;
+    a.ncol = gx * L.nc[2] * N;
+    a.inner = gx;
+    a.outer = gx * gy;
+    a.stride = gx;
+    line_launch(std::integral_constant<int, OP_INNER>{}, a, 1);
+  }
+  OpLineArgs a = args(DIM - 1);
+  a.p = DIM == 3 ? buf + 2 * nd : buf;
+  a.q = DIM == 3 ? buf + 3 * nd : buf + nd;
+  a.r = dst;
+  a.rhs = rhs;
+  a.ncol = DIM == 3 ? gx * gy : gx;
+  a.inner = a.ncol;
+  a.outer = 0;
+  a.stride = a.ncol;
+  if(rhs) line_launch(std::integral_constant<int, OP_RESIDUAL>{}, a, DIM - 1);
+  else line_launch(std::integral_constant<int, OP_LAST>{}, a, DIM - 1);
+}
+}  // namespace
+
+namespace
+{
+template<typename F>
+void for_size(int np, const F &f)
+{
+  switch(np)
+  {
+  case 2: f(std::integral_constant<int, 2>{}); break;
+  case 3: f(std::integral_constant<int, 3>{}); break;
+  case 4: f(std::integral_constant<int, 4>{}); break;
+  case 5: f(std::integral_constant<int, 5>{}); break;
+  case 6: f(std::integral_constant<int, 6>{}); break;
+  case 7: f(std::integral_constant<int, 7>{}); break;
+  case 8: f(std::integral_constant<int, 8>{}); break;
+  default: break;
+  }
+}
+}  // namespace
+
+void build_op_lines(tpss_operator &op, const tpss_layout &L, Penalty pen)
+{
+  for_size(L.np, [&](auto n) { build<decltype(n)::value>(op, L, pen); });
+}
+
+// false: not inside a stream capture before a first call outside it, and not when the device has no room
+// for the intermediate vectors (the cell-wise kernel then does without)
+bool op_lines_apply(tpss_operator &op, double *dst, const double *src, cudaStream_t s, const double *rhs)
+{
+  const tpss_layout &L = *op.layout;
+  OpLines &O = op.lines;
+  if(O.tables.n == 0) return false;
+  const size_t need = (size_t)L.n_dofs * (L.dim == 3 ? 4 : 2);
+  const ScratchUse use(O.order, s);
+  if(O.buf.n < need)
+  {
+    if(!use.may_allocate()) return false;
+    try
+    {
+      O.buf.resize(need);
+    }
+    catch(const Error &)
+    {
+      cudaGetLastError();
+      return false;
+    }
+  }
+  for_size(L.np, [&](auto n) {
+    if(L.dim == 2) run<2, decltype(n)::value>(op, O.buf.ptr, dst, src, s, rhs);
+    else run<3, decltype(n)::value>(op, O.buf.ptr, dst, src, s, rhs);
+  });
+  return true;
+}
+}  // namespace tpss

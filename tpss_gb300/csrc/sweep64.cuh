@@ -85,14 +85,6 @@ __device__ __forceinline__ int pencil_exponent(const double (&v)[N], bool fp64_o
   return zero ? 1023 : emax;
 }
 
-// y 2^ex as a double (ex keeps the result in the normal range)
-__device__ __forceinline__ double to_double(int64_t y, int ex)
-{
-  const double d = __ll2double_rn(y);
-  const int hi = y == 0 ? 0 : __double2hiint(d) + ex * (1 << 20);
-  return __hiloint2double(hi, __double2loint(d));
-}
-
 // S^T or S of one pencil v (FP64 values) into the thread's column col[m STRIDE] as FP64 values
 template<int N, bool FWD, int STRIDE>
 __device__ __forceinline__ void transform(const double (&v)[N], int64_t *col, const SweepTab &t, const int2 *slot, int e,
@@ -112,7 +104,7 @@ __device__ __forceinline__ void transform(const double (&v)[N], int64_t *col, co
   fd::fix_pass<N, FWD, STRIDE, 1>(c, slot, sy, [&](int, int m) { return fx::from_double(v[m], emax); });
   const int ex = emax - 1023 - 58 + 64 - F;
 #pragma unroll
-  for(int m = 0; m < N; ++m) out[m * STRIDE] = to_double(col[m * STRIDE], ex);
+  for(int m = 0; m < N; ++m) out[m * STRIDE] = fx::to_double(col[m * STRIDE], ex);
 }
 
 enum LineMode
@@ -242,7 +234,7 @@ __global__ void __launch_bounds__(kLineThreads, K1 <= 5 ? 6 : 4) line_kernel(Lin
           fd::fix_pass<N, false, BT, 1>(cp, s_tab, sy, [&](int, int m) { return col[m * BT]; });
           ex += 64 - F.y;
 #pragma unroll
-          for(int m = 0; m < N; ++m) cold[m * BT] = to_double(col[m * BT], ex);
+          for(int m = 0; m < N; ++m) cold[m * BT] = fx::to_double(col[m * BT], ex);
         }
       }
       if(v > c0)  // cell v - 1 is complete
