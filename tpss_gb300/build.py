@@ -25,7 +25,7 @@ FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", 
 
 UNITS = [
     ("setup.cu", []), ("eigen.cu", []), ("fixed_tab.cu", []), ("layout.cu", []), ("precond.cu", []),
-    ("operator.cu", []), ("sipg_lines.cu", []), ("mg.cu", []), ("diag.cu", []), ("stream3d.cu", []), ("mapped.cu", []), ("mapped_mf.cu", []), ("local.cu", []), ("mlp.cu", []), ("learned.cu", []), ("c0ip.cu", []),
+    ("operator.cu", []), ("sipg_lines.cu", []), ("transfer64.cu", []), ("mg.cu", []), ("diag.cu", []), ("stream3d.cu", []), ("mapped.cu", []), ("mapped_mf.cu", []), ("local.cu", []), ("mlp.cu", []), ("learned.cu", []), ("c0ip.cu", []),
     ("plane_inst.cu", ["-DPLANE_BZ=8"]), ("plane_inst.cu", ["-DPLANE_BZ=4"]),
     ("stream_k5.cu", ["-DK5_PART=0"]), ("stream_k5.cu", ["-DK5_PART=1"]),
     ("sweep64.cu", ["-DSWEEP_PART=0"]), ("sweep64.cu", ["-DSWEEP_PART=1"]), ("sweep64.cu", ["-DSWEEP_PART=2"]),

@@ -499,8 +499,9 @@ void extract_local_matrices(const tpss_layout &L, const tpss_operator &op, int64
 
 // operator and transfer (operator.cu)
 // dst = A src, or with rhs the residual dst = rhs - A src
+// cellwise: sipg_kernel also where the line-by-line form applies, with the rounding it has
 void operator_apply(tpss_operator *op, double *dst, const double *src, cudaStream_t s,
-                    const double *rhs = nullptr);
+                    const double *rhs = nullptr, bool cellwise = false);
 // line-by-line form of the FP64 product on a Cartesian level; false without tables or room for its
 // intermediate vectors (also while a stream is captured before the first product)
 void build_op_lines(tpss_operator &op, const tpss_layout &L, Penalty pen);
@@ -510,9 +511,19 @@ bool op_lines_apply(tpss_operator &op, double *dst, const double *src, cudaStrea
 // copy of the block-sparse matrix)
 void operator_apply_f32(tpss_operator *op, double *dst, const double *src, cudaStream_t s,
                         const double *rhs = nullptr);
-// single: FP32 arithmetic on the FP64 vectors (the transfers of a single-precision V-cycle)
+// FP64 arithmetic on the integer pipe (transfer64.cu); E_dev: the table of embedding_device
+void transfer_apply64(int dim, int k, const int *ncc, const double *E_dev, bool restrict_mode, double *coarse,
+                      double *fine, cudaStream_t s);
+// integer tables of degree np - 1, appended to the FP64 embeddings
+void append_transfer_tables(int np, std::vector<double> &buf);
+enum class TransferArith
+{
+  fp64,
+  fp64_tree,  // child by child, with the rounding that form has
+  single      // FP32 arithmetic on the FP64 vectors (the transfers of a single-precision V-cycle)
+};
 void transfer_apply(int dim, int k, const int *ncc, const double *E_dev, bool restrict_mode,
-                    double *coarse, double *fine, cudaStream_t s, bool single = false);
+                    double *coarse, double *fine, cudaStream_t s, TransferArith arith = TransferArith::fp64);
 
 // vector kernels (operator.cu)
 void vec_axpby(int64_t n, double a, const double *x, double b, double *y, cudaStream_t s);  // y = a x + b y

@@ -367,7 +367,8 @@ __device__ __forceinline__ void pencil_io(const T *in, T *out, const T *B, int p
 // along y (4) and E_bz along z (8) instead of 3 passes per child (24); restriction runs the
 // transposed tree (z: 8, y: 4, x: 2), summing the children on the way up.
 // T: arithmetic and shared-memory type (float for the transfers of a single-precision V-cycle:
-// FP64 vectors, each value converted once on the way in and out)
+// FP64 vectors, each value converted once on the way in and out; double next to smoothers in single
+// precision, the other FP64 transfers are those of transfer64.cuh)
 template<int DIM, int NP, bool RESTRICT, typename T>
 __global__ void __launch_bounds__(OpCfg<DIM, NP>::THREADS) transfer_kernel(TrArgs a)
 {
@@ -633,7 +634,7 @@ OpArgs<T> op_args(const tpss_operator &op, const T *src, double *dst, const doub
 }
 }  // namespace
 
-void operator_apply(tpss_operator *op, double *dst, const double *src, cudaStream_t s, const double *rhs)
+void operator_apply(tpss_operator *op, double *dst, const double *src, cudaStream_t s, const double *rhs, bool cellwise)
 {
   const tpss_layout &L = *op->layout;
   TPSS_REQUIRE(dst && src && dst != src, "operator: invalid vectors");
@@ -642,7 +643,7 @@ void operator_apply(tpss_operator *op, double *dst, const double *src, cudaStrea
     mapped_apply(*op, dst, src, s, rhs);
     return;
   }
-  if(op_lines_apply(*op, dst, src, s, rhs)) return;
+  if(!cellwise && op_lines_apply(*op, dst, src, s, rhs)) return;
   const OpArgs<double> a = op_args<double>(*op, src, dst, rhs);
   TPSS_DISPATCH_NP(L.dim, L.np, launch_sipg, a, s);
 }
@@ -665,8 +666,13 @@ void operator_apply_f32(tpss_operator *op, double *dst, const double *src, cudaS
 }
 
 void transfer_apply(int dim, int k, const int *ncc, const double *E_dev, bool restrict_mode,
-                    double *coarse, double *fine, cudaStream_t s, bool single)
+                    double *coarse, double *fine, cudaStream_t s, TransferArith arith)
 {
+  if(arith == TransferArith::fp64)
+  {
+    transfer_apply64(dim, k, ncc, E_dev, restrict_mode, coarse, fine, s);
+    return;
+  }
   TrArgs a;
   a.coarse = coarse;
   a.fine = fine;
@@ -677,7 +683,7 @@ void transfer_apply(int dim, int k, const int *ncc, const double *E_dev, bool re
     a.ncc[d] = d < dim ? ncc[d] : 1;
     a.n_coarse *= a.ncc[d];
   }
-  TPSS_DISPATCH_NP(dim, k + 1, launch_transfer, a, restrict_mode, single, s);
+  TPSS_DISPATCH_NP(dim, k + 1, launch_transfer, a, restrict_mode, arith == TransferArith::single, s);
 }
 
 void vec_axpby(int64_t n, double a, const double *x, double b, double *y, cudaStream_t s)
@@ -815,7 +821,8 @@ const double *embedding_device(int k)
   if(!t)
   {
     const Shape1D s = make_shape_1d(k);
-    const std::vector<double> E = embedding_1d(s);
+    std::vector<double> E = embedding_1d(s);
+    append_transfer_tables(k + 1, E);
     double *d = nullptr;
     TPSS_CUDA(cudaMalloc(&d, E.size() * sizeof(double)));
     TPSS_CUDA(cudaMemcpy(d, E.data(), E.size() * sizeof(double), cudaMemcpyHostToDevice));

@@ -931,7 +931,10 @@ void precond_vmult(tpss_precond *p, double *dst, const double *src, cudaStream_t
     {
       {
         ScopedTimer t(p, 0, s);
-        operator_apply(p->op, res, dst, s);
+        // In single precision the color kernels round this residual to FP32, where a last-bit difference at a
+        // rounding border becomes 6e-8 of the value: the cell-wise operator keeps those results to the bit
+        // (with the line-by-line one 5 of 8 sweeps over 10 x 11 x 12 cells, k = 3, differed, by up to 2e-9)
+        operator_apply(p->op, res, dst, s, nullptr, p->desc.precision == TPSS_FP32);
         vec_sub(L.n_dofs, src, res, s);  // res = src - A dst
       }
       ScopedTimer t(p, 1, s);

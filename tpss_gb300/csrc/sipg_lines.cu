@@ -4,6 +4,7 @@
 #include <map>
 #include <type_traits>
 
+#include "element_ext.h"
 #include "internal.h"
 #include "sipg_lines.cuh"
 
@@ -13,81 +14,9 @@ using namespace lines;
 
 namespace
 {
-// 1-D reference element in extended precision: the integers of the tables hold 62 bits, and the rounding
-// of the FP64 basis (some 1e-15 of an entry for high degrees) would be the operator's largest error.
-// mass and stiffness on [0, 1], derivatives at the upper end (those at the lower end mirror them)
-template<int N>
-struct Element
-{
-  long double mass[N][N], stiff[N][N], g[N];
-};
-
-template<int N>
-Element<N> make_element(const Shape1D &s)
-{
-  using R = long double;
-  // P_m and its derivative at z in (-1, 1)
-  auto legendre = [](int m, R z, R &p, R &dp) {
-    R p0 = 1, p1 = z;
-    for(int j = 2; j <= m; ++j)
-    {
-      const R p2 = ((2 * j - 1) * z * p1 - (j - 1) * p0) / j;
-      p0 = p1;
-      p1 = p2;
-    }
-    p = p1;
-    dp = m * (z * p1 - p0) / (z * z - 1);
-  };
-  // the FP64 points, one Newton step each (quadratic: twice as many digits), by symmetry in pairs
-  R x[N], qx[N], qw[N];
-  x[0] = 0;
-  x[N - 1] = 1;
-  for(int i = 0; i < N; ++i)
-  {
-    R z = 2 * (R)s.qx[i] - 1, p, dp;
-    legendre(N, z, p, dp);
-    z -= p / dp;
-    legendre(N, z, p, dp);
-    qx[i] = (1 + z) / 2;
-    qw[i] = 1 / ((1 - z * z) * dp * dp);
-    if(i == 0 || i == N - 1) continue;
-    z = 2 * (R)s.nodes[i] - 1;
-    legendre(N - 1, z, p, dp);
-    z -= dp * (1 - z * z) / (2 * z * dp - (R)(N - 1) * N * p);
-    x[i] = (1 + z) / 2;
-  }
-  auto lagrange = [&](R at, R(&v)[N], R(&d)[N]) {
-    for(int i = 0; i < N; ++i)
-    {
-      v[i] = 1;
-      d[i] = 0;
-      for(int j = 0; j < N; ++j)
-      {
-        if(j == i) continue;
-        d[i] = (d[i] * (at - x[j]) + v[i]) / (x[i] - x[j]);
-        v[i] *= (at - x[j]) / (x[i] - x[j]);
-      }
-    }
-  };
-  Element<N> e{};
-  R v[N], d[N];
-  for(int q = 0; q < N; ++q)
-  {
-    lagrange(qx[q], v, d);
-    for(int i = 0; i < N; ++i)
-      for(int j = 0; j < N; ++j)
-      {
-        e.mass[i][j] += v[i] * v[j] * qw[q];
-        e.stiff[i][j] += d[i] * d[j] * qw[q];
-      }
-  }
-  lagrange(1, v, e.g);
-  return e;
-}
-
 // Table of one cell width h (layout OpTab<N>)
 template<int N>
-void fill_table(const Element<N> &s, double h, long double sigma, std::vector<long double> &t)
+void fill_table(const ext::Element<N> &s, double h, long double sigma, std::vector<long double> &t)
 {
   using T = OpTab<N>;
   constexpr int H = T::H, HE = T::HE;
@@ -154,7 +83,7 @@ template<int N>
 void build(tpss_operator &op, const tpss_layout &L, Penalty pen)
 {
   using T = OpTab<N>;
-  const Element<N> s = make_element<N>(make_shape_1d(L.k));
+  const ext::Element<N> s(make_shape_1d(L.k));
   const double gamma = double(L.k) * (L.k + 1);
   OpLines &O = op.lines;
   // per direction: [integer tables][FP64 tables][sigma: 3 per cell][exponents: 3 per width][width per cell]
@@ -182,10 +111,7 @@ void build(tpss_operator &op, const tpss_layout &L, Penalty pen)
         for(int i = 0; i < T::SIZE; ++i)
         {
           const int f = i < T::CE ? F[0] : i < T::TE ? F[1] : F[2];
-          const int64_t v = std::llrint(std::ldexp(t[i], f));
-          const int32_t lo = (int32_t)(uint32_t)(uint64_t)v;
-          const int32_t hi = (int32_t)((v - lo) >> 32);
-          ti.push_back((int64_t)((uint64_t)(uint32_t)hi << 32 | (uint32_t)lo));
+          ti.push_back(ext::limbs(t[i], f));
         }
         t64.insert(t64.end(), t.begin(), t.end());
         exps.insert(exps.end(), F, F + 3);
