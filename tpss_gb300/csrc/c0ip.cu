@@ -22,7 +22,10 @@
 #include <algorithm>
 #include <cmath>
 #include <map>
+#include <type_traits>
 
+#include "c0ip_band.cuh"
+#include "element_ext.h"
 #include "internal.h"
 
 namespace tpss
@@ -374,6 +377,10 @@ struct C0ipLevel
 {
   int nc = 0, n = 0;  // cells per direction, interior nodes per direction (nc k - 1)
   tpss::DeviceBuffer<double> bandM, bandL, bandB;
+  // integer rows per class of cells (c0ip_band.cuh); n_cls = 0: too many classes
+  tpss::DeviceBuffer<int64_t> band_tab;
+  tpss::DeviceBuffer<int32_t> band_cls;
+  int n_cls = 0, FM = 0, FL = 0, FB = 0;
   std::vector<int64_t> color_start;  // 5 entries
   tpss::DeviceBuffer<int32_t> vertex, key;
   tpss::DeviceBuffer<double> tab64;
@@ -450,6 +457,92 @@ std::vector<double> cholesky_inv(const std::vector<double> &A, int N)
 // 1-D key of a patch position: bit 0 touches the lower boundary, bit 1 the upper one
 int key_1d(int v, int nc) { return (v == 1 ? 1 : 0) | (v == nc - 1 ? 2 : 0); }
 
+template<typename F>
+void for_degree(int k, const F &f)
+{
+  switch(k)
+  {
+  case 2: f(std::integral_constant<int, 2>{}); break;
+  case 3: f(std::integral_constant<int, 3>{}); break;
+  case 4: f(std::integral_constant<int, 4>{}); break;
+  case 5: f(std::integral_constant<int, 5>{}); break;
+  case 6: f(std::integral_constant<int, 6>{}); break;
+  case 7: f(std::integral_constant<int, 7>{}); break;
+  default: break;
+  }
+}
+
+// Integer rows of the operator's bands (c0ip_band.cuh), one set per class of cells with equal rows. None
+// (n_cls = 0: the kernels by node run) when there are more classes than a launch holds or when an entry that
+// the integer kernels leave out is not zero.
+template<int K>
+void build_band_tables(C0ipLevel &L, int nc, const std::vector<double> &M, const std::vector<double> &Lm,
+                       const std::vector<double> &B)
+{
+  using T = band::Tab<K>;
+  constexpr int W = 4 * K + 1;
+  const int n = L.n;
+  auto exponent = [&](const std::vector<double> &A) {
+    double mx = 0.0;
+    for(int i = 0; i < n; ++i)
+    {
+      double s = 0.0;
+      for(int j = 0; j < W; ++j) s += std::fabs(A[(size_t)i * W + j]);
+      mx = std::max(mx, s * (1.0 + 1e-14));
+    }
+    int e = 0;
+    std::frexp(mx, &e);
+    return 62 - e;
+  };
+  L.FM = exponent(M);
+  L.FL = exponent(Lm);
+  L.FB = exponent(B);
+  std::map<std::vector<int64_t>, int> ids;
+  std::vector<int32_t> cls(nc);
+  std::vector<int64_t> tab;
+  for(int c = 0; c < nc; ++c)
+  {
+    // most cells have the rows of the one before
+    const size_t at = (size_t)(c * K - 1) * W, len = (size_t)K * W;
+    auto as_before = [&](const std::vector<double> &A) { return std::equal(&A[at], &A[at] + len, &A[at - len]); };
+    if(c > 1 && as_before(M) && as_before(Lm) && as_before(B))
+    {
+      cls[c] = cls[c - 1];
+      continue;
+    }
+    std::vector<int64_t> t(T::SIZE, 0);
+    for(int r = 0; r < K; ++r)
+    {
+      const int i = c * K + r - 1;
+      if(i < 0) continue;
+      // window entry j of a row: column c K - (2 K or K) + j, of which the kernel contracts [first, first + len)
+      auto fill = [&](const std::vector<double> &A, int f, int half, int first, int len, int at) {
+        for(int o = -2 * K; o <= 2 * K; ++o)
+        {
+          const double v = A[(size_t)i * W + o + 2 * K];
+          const int j = r + o + half;
+          if(j >= first && j < first + len) t[at + j - first] = ext::limbs(v, f);
+          else if(v != 0.0) return false;
+        }
+        return true;
+      };
+      const int row = T::R + (r - 1) * T::RS;
+      const bool ok = r == 0 ? fill(B, L.FB, 2 * K, 0, T::WB, 0) && fill(M, L.FM, K, 0, T::WM, T::M0) &&
+                                 fill(Lm, L.FL, K, 0, T::WM, T::L0)
+                             : fill(B, L.FB, 2 * K, K, T::NB, row) && fill(M, L.FM, K, K, T::NM, row + T::RM) &&
+                                 fill(Lm, L.FL, K, K, T::NM, row + T::RL);
+      if(!ok) return;
+    }
+    const auto it = ids.emplace(t, (int)ids.size());
+    if(it.second) tab.insert(tab.end(), t.begin(), t.end());
+    cls[c] = it.first->second;
+    if(ids.size() > band::kMaxClasses) return;
+  }
+  L.band_tab.upload(tab.data(), tab.size());
+  L.band_cls.upload(cls.data(), cls.size());
+  L.n_cls = (int)ids.size();
+}
+
 void build_level(tpss_c0ip &c, C0ipLevel &L, const Poly1D &poly, int nc)
 {
   const tpss_c0ip_desc &d = c.desc;
@@ -459,9 +552,11 @@ void build_level(tpss_c0ip &c, C0ipLevel &L, const Poly1D &poly, int nc)
   Band1D M, Lm, B;
   global_1d(poly, nc, d.ip_factor, M, Lm, B);
   if(d.problem == TPSS_Q_POISSON) B = Lm;  // A = M (x) L + L (x) M
-  L.bandM.upload(to_band(M, na, bw).data(), (size_t)L.n * (2 * bw + 1));
-  L.bandL.upload(to_band(Lm, na, bw).data(), (size_t)L.n * (2 * bw + 1));
-  L.bandB.upload(to_band(B, na, bw).data(), (size_t)L.n * (2 * bw + 1));
+  const std::vector<double> hM = to_band(M, na, bw), hL = to_band(Lm, na, bw), hB = to_band(B, na, bw);
+  L.bandM.upload(hM.data(), hM.size());
+  L.bandL.upload(hL.data(), hL.size());
+  L.bandB.upload(hB.data(), hB.size());
+  for_degree(k, [&](auto kk) { build_band_tables<decltype(kk)::value>(L, nc, hM, hL, hB); });
   // patches, colors (vx % 2) + 2 (vy % 2), lexicographic inside a color
   std::vector<int32_t> vert, key;
   L.color_start.assign(1, 0);
@@ -599,9 +694,44 @@ void build_transfer(tpss_c0ip &c, C0ipLevel &F, const Poly1D &poly, int ncc)
   F.tmp.resize((size_t)nf * nf);
 }
 
-void op_apply(const tpss_c0ip &c, const C0ipLevel &L, double *dst, const double *src, cudaStream_t s)
+// by_node: the FP64 kernels also where the integer ones apply, with the rounding they have: a cycle with
+// smoothers in single precision rounds the residual to FP32, where a last-bit difference can become 6e-8
+void op_apply(const tpss_c0ip &c, const C0ipLevel &L, double *dst, const double *src, cudaStream_t s, bool by_node)
 {
   const int64_t N = (int64_t)L.n * L.n;
+  if(L.n_cls > 0 && !by_node)
+  {
+    for_degree(c.desc.degree, [&](auto kk) {
+      constexpr int K = decltype(kk)::value;
+      band::BandArgs a{};
+      a.M = L.bandM.ptr;
+      a.L = L.bandL.ptr;
+      a.B = L.bandB.ptr;
+      a.tab = reinterpret_cast<const int2 *>(L.band_tab.ptr);
+      a.cls = L.band_cls.ptr;
+      a.n_cls = L.n_cls;
+      a.n = L.n;
+      a.nc = L.nc;
+      a.FM = L.FM;
+      a.FL = L.FL;
+      a.FB = L.FB;
+      a.mixed = c.mixed;
+      const size_t smem = (size_t)L.n_cls * band::Tab<K>::SIZE * 8;
+      const unsigned grid = (unsigned)(((int64_t)L.nc * L.n + 127) / 128);
+      a.a = src;
+      a.ra = L.tm.ptr;
+      a.rb = L.tl.ptr;
+      a.rc = L.tb.ptr;
+      band::band_x_kernel<K><<<grid, 128, smem, s>>>(a);
+      a.a = L.tm.ptr;
+      a.b = L.tl.ptr;
+      a.c = L.tb.ptr;
+      a.ra = dst;
+      band::band_y_kernel<K><<<grid, 128, smem, s>>>(a);
+    });
+    TPSS_CUDA(cudaGetLastError());
+    return;
+  }
   c0ip_x_kernel<<<grid_for_c(N), 256, 0, s>>>(src, L.n, c.bw, L.bandM.ptr, L.bandL.ptr, L.bandB.ptr,
                                              L.tm.ptr, L.tl.ptr, L.tb.ptr);
   c0ip_y_kernel<<<grid_for_c(N), 256, 0, s>>>(L.tm.ptr, L.tl.ptr, L.tb.ptr, L.n, c.bw, L.bandM.ptr,
@@ -734,12 +864,12 @@ void vcycle(tpss_c0ip &c, int l, cudaStream_t s)
   }
   C0ipLevel &Cl = c.lv[l - 1];
   smooth(c, L, L.x.ptr, L.b.ptr, s);
-  op_apply(c, L, L.t.ptr, L.x.ptr, s);
+  op_apply(c, L, L.t.ptr, L.x.ptr, s, c.desc.precision == TPSS_FP32);
   vec_axpby(N, 1.0, L.b.ptr, -1.0, L.t.ptr, s);  // t = b - A x
   restrict_to(L, Cl, Cl.b.ptr, L.t.ptr, s);
   vcycle(c, l - 1, s);
   prolongate_add(L, Cl, L.x.ptr, Cl.x.ptr, s);
-  op_apply(c, L, L.t.ptr, L.x.ptr, s);
+  op_apply(c, L, L.t.ptr, L.x.ptr, s, c.desc.precision == TPSS_FP32);
   vec_axpby(N, 1.0, L.b.ptr, -1.0, L.t.ptr, s);
   smooth(c, L, L.r.ptr, L.t.ptr, s);
   vec_axpby(N, 1.0, L.r.ptr, 1.0, L.x.ptr, s);  // x += P (b - A x)
@@ -826,7 +956,7 @@ extern "C" int tpss_c0ip_operator_vmult(tpss_c0ip *c, int level, double *dst, co
     TPSS_REQUIRE(c && dst && src && dst != src, "invalid argument");
     const int nl = (int)c->lv.size(), l = level < 0 ? nl - 1 : level;
     TPSS_REQUIRE(l < nl, "invalid level");
-    op_apply(*c, c->lv[l], dst, src, as_stream(stream));
+    op_apply(*c, c->lv[l], dst, src, as_stream(stream), false);
   });
 }
 
@@ -905,7 +1035,7 @@ extern "C" int tpss_c0ip_cg_solve(tpss_c0ip *c, double *u, const double *f, doub
       const unsigned vg = (unsigned)std::min<int64_t>((N + 255) / 256, (int64_t)num_sms() * 8);
       for(it = 1; it <= max_iter; ++it)
       {
-        op_apply(*c, T, c->cAp.ptr, c->cp.ptr, s);
+        op_apply(*c, T, c->cAp.ptr, c->cp.ptr, s, c->desc.precision == TPSS_FP32);
         vec_dot(N, c->cp.ptr, c->cAp.ptr, c->partial.ptr, sc + 1, s);  // pAp
         c0ip_cg_scalars<<<1, 1, 0, s>>>(sc, 0);                          // alpha = rz / pAp
         c0ip_axpby_dev<<<vg, 256, 0, s>>>(N, sc + 4, c->cp.ptr, sc + 7, u);
