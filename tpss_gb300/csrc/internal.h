@@ -527,7 +527,6 @@ void transfer_apply(int dim, int k, const int *ncc, const double *E_dev, bool re
 
 // vector kernels (operator.cu)
 void vec_axpby(int64_t n, double a, const double *x, double b, double *y, cudaStream_t s);  // y = a x + b y
-void vec_sub(int64_t n, const double *a, double *y, cudaStream_t s);  // y = a - y
 // dot products: partial sums into `partial` (device, >= dot_partials()), final into out (device)
 int dot_partials();
 void vec_dot(int64_t n, const double *x, const double *y, double *partial, double *out,

@@ -556,12 +556,6 @@ __global__ void axpby_kernel(int64_t n, double a, const double *__restrict__ x, 
     y[i] = a * x[i] + b * y[i];
 }
 
-__global__ void sub_kernel(int64_t n, const double *__restrict__ a, double *__restrict__ y)
-{
-  for(int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    y[i] = a[i] - y[i];
-}
-
 __global__ void d2f_kernel(int64_t n, const double *__restrict__ x, float *__restrict__ y)
 {
   for(int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
@@ -689,12 +683,6 @@ void transfer_apply(int dim, int k, const int *ncc, const double *E_dev, bool re
 void vec_axpby(int64_t n, double a, const double *x, double b, double *y, cudaStream_t s)
 {
   axpby_kernel<<<vec_grid(n), 256, 0, s>>>(n, a, x, b, y);
-  TPSS_CUDA(cudaGetLastError());
-}
-
-void vec_sub(int64_t n, const double *a, double *y, cudaStream_t s)
-{
-  sub_kernel<<<vec_grid(n), 256, 0, s>>>(n, a, y);
   TPSS_CUDA(cudaGetLastError());
 }
 

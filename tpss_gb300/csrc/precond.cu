@@ -934,8 +934,7 @@ void precond_vmult(tpss_precond *p, double *dst, const double *src, cudaStream_t
         // In single precision the color kernels round this residual to FP32, where a last-bit difference at a
         // rounding border becomes 6e-8 of the value: the cell-wise operator keeps those results to the bit
         // (with the line-by-line one 5 of 8 sweeps over 10 x 11 x 12 cells, k = 3, differed, by up to 2e-9)
-        operator_apply(p->op, res, dst, s, nullptr, p->desc.precision == TPSS_FP32);
-        vec_sub(L.n_dofs, src, res, s);  // res = src - A dst
+        operator_apply(p->op, res, dst, s, src, p->desc.precision == TPSS_FP32);  // res = src - A dst
       }
       ScopedTimer t(p, 1, s);
       apply_color(p, seq[i], dst, res, s);
@@ -1125,8 +1124,7 @@ void smoother_steps(tpss_smoother *sm, double *x, const double *b, cudaStream_t 
   if(sm->tmp.n < (size_t)n) sm->tmp.resize(n);
   for(int k = 0; k < sm->n_steps; ++k)
   {
-    operator_apply(sm->op, sm->residual.ptr, x, s);  // r = A x
-    vec_sub(n, b, sm->residual.ptr, s);              // r = b - A x
+    operator_apply(sm->op, sm->residual.ptr, x, s, b);  // r = b - A x
     precond_vmult(sm->p, sm->tmp.ptr, sm->residual.ptr, s);
     vec_axpby(n, sm->damping, sm->tmp.ptr, 1.0, x, s);  // x += damping P r
   }
