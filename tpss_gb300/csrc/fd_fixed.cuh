@@ -210,7 +210,7 @@ __device__ __forceinline__ unsigned fix_pass(int64_t *const (&data)[NPT], const 
   return mag;
 }
 
-// A pencil's values v[i STRIDE] times positive factors r(i), which may span many orders of magnitude:
+// A pencil's values v[i STRIDE] times positive factors r(i) = m 2^q (in limbs), which may span many orders of magnitude:
 // the products are floating point per value first and then share one exponent, with which the
 // largest has 59 bits. Returns that exponent less 61 (and whether any product is not zero).
 template<int N, int STRIDE, typename R>
@@ -223,7 +223,7 @@ __device__ __forceinline__ int scale_by_reciprocals(int64_t *v, const R &r, bool
   for(int i = 0; i < N; ++i)
   {
     int mh, ml;
-    fx::split_positive(r(i), mh, ml, qe[i]);
+    r(i, mh, ml, qe[i]);
     y[i] = fx::mul_m61(v[i * STRIDE], mh, ml);
     e0 = max(e0, qe[i]);
   }
@@ -512,7 +512,12 @@ __global__ void __maxnreg__((FixCfg<DIM, NCP, K1>::REGS))
         }
         bool any;
         const int e59 = scale_by_reciprocals<N, LSTR>(
-          v, [&](int i) { return rt ? __ldg(rt + i * NPENCIL) : 1.0 / (lsum + lamL[i]); }, any);
+          v,
+          [&](int i, int &mh, int &ml, int &q) {
+            if(rt) fx::split_positive(__ldg(rt + i * NPENCIL), mh, ml, q);
+            else fx::reciprocal(lsum + lamL[i], mh, ml, q);
+          },
+          any);
         g[j] = e59;
         if(any) xb = max(xb, (unsigned)(e59 + 59 + kExpBias));
       }
