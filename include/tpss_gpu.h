@@ -235,8 +235,9 @@ int tpss_precond_vmult_static_scratch(tpss_precond *p, double *dst, const double
 
 /* Autotuner (no counterpart in the reference): times every work decomposition of the smoother
  * kernel for this level (for the column-streamed kernel: pencils per thread, vertex layers per
- * work item and, for degree 4, pencil or plane passes; for the per-color kernel, which serves 2D, cell patches, FP64, k > 4 and the
- * multiplicative smoother: 1, 2 or 4 times its base number of patches per CTA, as far as 512
+ * work item and, for degree 4, pencil or plane passes; the FP64 additive smoother on vertex patches of a
+ * Cartesian level goes direction by direction and has one; for the per-color kernel, which serves 2D, cell patches, k > 4,
+ * distorted levels and the multiplicative smoother: 1, 2 or 4 times its base number of patches per CTA, as far as 512
  * threads and 200 KB of shared memory allow) on the caller's vectors, `reps` applications each,
  * and keeps the fastest for later vmult calls.  On return dst = P src, *chosen is the selected variant, ms_per_variant (optional,
  * >= 8 entries) the measured milliseconds per application and *n_variants their count (1 when the
