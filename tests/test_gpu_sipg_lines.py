@@ -45,7 +45,9 @@ def apply(op, src, cuda):
 # block of 128 lines; long lines (several segments); every degree
 SIZES = [(2, 1, (41, 2)), (2, 2, (13, 1)), (2, 3, (10, 33)), (2, 4, (1, 1)), (2, 5, (7, 70)), (2, 6, (6, 9)), (2, 7, (5, 300)),
          (3, 1, (21, 3, 2)), (3, 2, (14, 5, 1)), (3, 3, (9, 2, 7)), (3, 4, (8, 3, 40)), (3, 4, (1, 1, 1)), (3, 5, (6, 1, 3)),
-         (3, 6, (3, 4, 2)), (3, 7, (6, 2, 2))]
+         (3, 6, (3, 4, 2)), (3, 7, (6, 2, 2)),
+         # the lower degrees above take the cell-wise kernel on levels of that size; these do not
+         (2, 1, (41, 830)), (2, 2, (13, 320)), (3, 1, (21, 40, 30)), (3, 2, (14, 31, 10)), (3, 3, (9, 11, 9)), (3, 4, (1, 10, 9))]
 
 
 @pytest.mark.parametrize("dim,k,nc", SIZES)
@@ -59,7 +61,7 @@ def test_sizes_and_widths(tpss, oracle, cuda, dim, k, nc):
             assert rel_err(apply(op, src * scale, cuda) / scale, ref) <= 1e-12, (h is None, scale)
 
 
-@pytest.mark.parametrize("dim,k,nc", [(2, 3, (11, 6)), (3, 2, (5, 6, 4))])
+@pytest.mark.parametrize("dim,k,nc", [(2, 3, (11, 6)), (3, 2, (5, 6, 4)), (3, 2, (15, 17, 17))])
 def test_cell_order_and_penalty(tpss, oracle, cuda, dim, k, nc):
     n_cells, cd = int(np.prod(nc)), (k + 1) ** dim
     cells = np.random.Generator(np.random.Philox(5)).permutation(n_cells).astype(np.int64) * cd
@@ -70,7 +72,7 @@ def test_cell_order_and_penalty(tpss, oracle, cuda, dim, k, nc):
     assert rel_err(apply(op, src, cuda), ref) <= 1e-12
 
 
-@pytest.mark.parametrize("dim,k,nc", [(2, 4, (9, 7)), (3, 3, (5, 4, 6))])
+@pytest.mark.parametrize("dim,k,nc", [(2, 4, (9, 7)), (3, 3, (5, 4, 6)), (3, 3, (10, 9, 10))])
 def test_range_zeros_and_nan(tpss, oracle, cuda, dim, k, nc):
     cd = (k + 1) ** dim
     n = int(np.prod(nc)) * cd

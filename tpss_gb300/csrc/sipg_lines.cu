@@ -235,13 +235,26 @@ void build_op_lines(tpss_operator &op, const tpss_layout &L, Penalty pen)
   for_size(L.np, [&](auto n) { build<decltype(n)::value>(op, L, pen); });
 }
 
-// false: not inside a stream capture before a first call outside it, and not when the device has no room
+// Whether the passes are faster than the cell-wise kernel. On small levels both are latency: the passes take 12.4
+// (2D) and 18.6 us (3D) whatever the degree, the cell-wise kernel 9, 11.5 and 14.5 us for k = 1, 2, 3 in 2D and
+// 10.4, 13.8, 14.8, 18 and 21 us for k = 1 .. 5 in 3D; beyond that its multiply-adds cost 1.7 us per million
+// (2 per clock and SM), the passes' about 0.28 of that. The lines below are where the two meet
+// (measured equal: 2D k = 1 160^2 cells, 14.4 and 14.5 us; 3D k = 4 6^3, 18.6 and 19.1)
+bool lines_pay(const tpss_layout &L)
+{
+  static const double from[2][8] = {{0, 4.6, 1.4, 0, 0, 0, 0, 0}, {0, 11.3, 7.8, 4.3, 0.8, 0, 0, 0}};
+  const double n = L.np, cells = (double)L.nc[0] * L.nc[1] * (L.dim == 3 ? L.nc[2] : 1);
+  const double fma = L.dim == 2 ? n * (4 * n * n + 4 * (2 * n + 2)) : n * n * (8 * n * n + 6 * (2 * n + 2));
+  return cells * fma * 1.7e-6 >= from[L.dim - 2][L.k];
+}
+
+// false: where the cell-wise kernel is faster, not inside a stream capture before a first call outside it, and not when the device has no room
 // for the intermediate vectors (the cell-wise kernel then does without)
 bool op_lines_apply(tpss_operator &op, double *dst, const double *src, cudaStream_t s, const double *rhs)
 {
   const tpss_layout &L = *op.layout;
   OpLines &O = op.lines;
-  if(O.tables.n == 0) return false;
+  if(O.tables.n == 0 || !lines_pay(L)) return false;
   const size_t need = (size_t)L.n_dofs * (L.dim == 3 ? 4 : 2);
   const ScratchUse use(O.order, s);
   if(O.buf.n < need)
