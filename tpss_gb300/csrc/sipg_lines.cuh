@@ -272,6 +272,7 @@ __device__ __forceinline__ void special_faces(const double *sg, bool below, bool
 
 // ---- y and last pass: one thread per line and segment
 constexpr int kOpThreads = 128;
+constexpr int kMaxSegments = 65535;  // a grid's second dimension (a longer line gets longer segments)
 
 enum OpLineMode
 {
@@ -392,7 +393,8 @@ __global__ void __launch_bounds__(OpXCfg<DIM, N>::THREADS) op_x_kernel(OpLineArg
   double *s_r = s_tr + 2 * P, *s_m = s_r + N * CS;
   int64_t *s_row = reinterpret_cast<int64_t *>(s_m + N * CS);
   const int tid = threadIdx.x, lane = tid % 32, warp = tid / 32, nx = a.nc[0];
-  const int ng = a.nc[1] * (DIM == 3 ? a.nc[2] : 1), g0 = blockIdx.x * C::XG, x0 = blockIdx.y * XC;
+  const int ng = a.nc[1] * (DIM == 3 ? a.nc[2] : 1), groups = (ng + C::XG - 1) / C::XG;
+  const int g0 = blockIdx.x % groups * C::XG, x0 = blockIdx.x / groups * XC;
   const int64_t gx_n = (int64_t)nx * N;
   const int w0 = a.width[x0] & ~kSpecial;
   // one table serves the tile when its cells have the same width
