@@ -16,7 +16,7 @@
 // t+ = (sigma_b - 2 sigma) u - t; unequal widths shift t+ by the difference of the penalties.
 // All contractions run in even/odd form with integers, one exponent per pencil (fixed64.cuh).
 //
-// Measured, 64^3 cells, k = 4 (32.8M DoFs): 905 us (x 366, y 289, last 244) against sipg_kernel's
+// Measured, 64^3 cells, k = 4 (32.8M DoFs): 953 us (x 396, y 303, last 252) against sipg_kernel's
 // 3,168 us, whose FP64 pipe is busy throughout. The vectors in between cost 2.4 GB of traffic in all
 // (0.36 ms at the copy rate), which the cell-wise kernel does not have; issue slots (56 % busy) and the
 // 32-bit multiplier (46 to 55 %) bound the passes. Of the conversions back to FP64 the results' use the
@@ -63,8 +63,8 @@ struct OpLineArgs
 
 // marks a cell with a face at the boundary or to a cell of another width: only these need the
 // penalties in FP64. Kept behind one branch, since the compiler otherwise predicates the corrections and
-// runs them for every cell (27 FP64 instructions per pencil instead of 7; the y pass of the level below
-// took 376 us so, and takes 289)
+// runs them for every cell (27 FP64 instructions per pencil instead of 7; the y pass of the level above
+// took 376 us so, and 289 without)
 constexpr int32_t kSpecial = 1 << 30;
 
 __device__ __forceinline__ double negated(double v)
@@ -109,22 +109,27 @@ __device__ __forceinline__ void split_parts(const double (&u)[N], int emax, int 
 // One pencil of a cell. In: q (and p) of the cell, the neighbours' face values uL, uR. Out: r without
 // the neighbours' traces, m, and the cell's traces towards its lower (tl) and upper (tu) neighbour.
 // PARTS: 0 traces only, 1 everything.
-template<int N, bool HAS_P, bool WANT_M, int PARTS>
+// The unit of q's integers is that of q alone: a larger value in a neighbour neither costs the traces and m,
+// which do not depend on it, any bits, nor makes them differ between a cell and its copy at the end of a tile
+// or segment. A face value more than two binades above q enters r in FP64 instead; it is rare and read once more
+// there (again: sets uL, uR), since the registers that would keep it cost 15 % of the passes' time (64^3 cells, k = 4:
+// 1,106 us; 953 so; 903 with one unit for q and the face values).
+template<int N, bool HAS_P, bool WANT_M, int PARTS, typename Again>
 __device__ __forceinline__ void cell_pencil(const int2 *__restrict__ tab, const double *__restrict__ tab64, int FM, int FC,
                                             int FT, const double (&p)[N], const double (&q)[N], double uL, double uR,
-                                            double (&r)[N], double (&m)[N], double &tl, double &tu)
+                                            double (&r)[N], double (&m)[N], double &tl, double &tu, const Again &again)
 {
   using T = OpTab<N>;
   constexpr int H = T::H, HE = T::HE;
-  unsigned hq = 0, lq = 0, hp = 0, lp = 0;
+  unsigned hq = 0, lq = 0, hn = 0, ln = 0, hp = 0, lp = 0;
   magnitude<N>(q, hq, lq);
   if constexpr(PARTS)
   {
     const double nb[2] = {uL, uR};
-    magnitude<2>(nb, hq, lq);
+    magnitude<2>(nb, hn, ln);
     if constexpr(HAS_P) magnitude<N>(p, hp, lp);
   }
-  if(out_of_range(hq, lq) || (PARTS && HAS_P && out_of_range(hp, lp)))
+  if(out_of_range(hq, lq) || (PARTS && (out_of_range(hn, ln) || (HAS_P && out_of_range(hp, lp)))))
   {
     // FP64, rolled (on copies, so that the values above stay in registers)
     double u[N], v[N], rr[N], mm[N];
@@ -183,7 +188,8 @@ __device__ __forceinline__ void cell_pencil(const int2 *__restrict__ tab, const 
     }
     return;
   }
-  const int eq = hq == 0 ? 1023 : (int)(hq >> 20), ep = hp == 0 ? 1023 : (int)(hp >> 20);
+  // (a zero pencil takes the unit of its neighbours)
+  const int en = (int)(hn >> 20), eq = hq != 0 ? (int)(hq >> 20) : hn != 0 ? en : 1023, ep = hp == 0 ? 1023 : (int)(hp >> 20);
   // limbs of the even parts and s, and of the odd parts and d
   int eh[1][HE + 1], el[1][HE + 1], oh[1][H + 1], ol[1][H + 1];
   split_parts<N>(q, eq, eh, el, oh, ol);
@@ -197,15 +203,17 @@ __device__ __forceinline__ void cell_pencil(const int2 *__restrict__ tab, const 
   }
   if constexpr(PARTS)
   {
+    // up to two binades above q the one product that a row has with them stays within the accumulators
+    const bool far = en > eq + 2;
     {
-      const int64_t lo = fx::from_double(uL, eq), hi = fx::from_double(uR, eq);
+      const int64_t lo = far ? 0 : fx::from_double(uL, eq + 2) << 2, hi = far ? 0 : fx::from_double(uR, eq + 2) << 2;
       fx::split(hi + lo, eh[0][HE], el[0][HE]);
       fx::split(hi - lo, oh[0][H], ol[0][H]);
     }
     int ph[1][HE + 1], pl[1][HE + 1], sh[1][H + 1], sl[1][H + 1];
     if constexpr(HAS_P) split_parts<N>(p, ep, ph, pl, sh, sl);
     // the two contributions to r come to the coarser of their units (a zero one has none)
-    const int u2 = ep - 1023 - 58 + 64 - FM, u1 = HAS_P && hq == 0 ? u2 : uq - FC;
+    const int u2 = ep - 1023 - 58 + 64 - FM, u1 = HAS_P && (hq | hn) == 0 ? u2 : uq - FC;
     const int U = HAS_P && hp != 0 ? max(u1, u2) : u1;
     auto even = [&](int i) {
       int64_t a[1];
@@ -239,6 +247,18 @@ __device__ __forceinline__ void cell_pencil(const int2 *__restrict__ tab, const 
       r[N - 1 - i] = fx::to_double(e - o, U);
     }
     if constexpr(N % 2 == 1) r[H] = fx::to_double(even(H), U);
+    if(far)
+    {
+      again(uL, uR);
+      const double s = uR + uL, d = uR - uL;
+#pragma unroll
+      for(int i = 0; i < HE; ++i)
+      {
+        const double e = tab64[T::CE + i * T::LCE + HE] * s, o = i < H ? tab64[T::CO + i * T::LCO + H] * d : 0.0;
+        r[i] += e + o;
+        if(i < H) r[N - 1 - i] += e - o;
+      }
+    }
     if constexpr(WANT_M)
     {
 #pragma unroll
@@ -281,8 +301,16 @@ enum OpLineMode
   OP_RESIDUAL,  // the same, dst = rhs - result
 };
 
+// registers per thread: what the passes need without the rare branch of cell_pencil (the compiler, left alone, takes up to 20
+// more for it, and an SM holds a block or two fewer)
+constexpr int line_regs(int n, bool last)
+{
+  constexpr int to[9] = {0, 0, 56, 72, 64, 80, 88, 104, 112}, in[9] = {0, 0, 64, 72, 64, 96, 112, 128, 128};
+  return last ? to[n] : in[n];
+}
+
 template<int DIM, int N, int MODE>
-__global__ void __launch_bounds__(kOpThreads) op_line_kernel(OpLineArgs a)
+__global__ void __maxnreg__((line_regs(N, MODE != OP_INNER))) op_line_kernel(OpLineArgs a)
 {
   using T = OpTab<N>;
   constexpr bool LAST = MODE != OP_INNER;
@@ -333,11 +361,15 @@ __global__ void __launch_bounds__(kOpThreads) op_line_kernel(OpLineArgs a)
 #pragma unroll
       for(int i = 0; i < N; ++i) pv[i] = p[(at + i) * a.stride];
       const double uL = x > 0 ? face : negated(qv[0]), uR = x + 1 < n ? q[(at + N) * a.stride] : negated(qv[N - 1]);
-      cell_pencil<N, true, !LAST, 1>(s_tab, t64, FM, FC, FT, pv, qv, uL, uR, r, m, tl, tu);
+      cell_pencil<N, true, !LAST, 1>(s_tab, t64, FM, FC, FT, pv, qv, uL, uR, r, m, tl, tu, [&](double &lo, double &hi) {
+        const double *f = q + at * a.stride;
+        lo = x > 0 ? f[-a.stride] : negated(f[0]);
+        hi = x + 1 < n ? f[N * a.stride] : negated(f[(N - 1) * a.stride]);
+      });
       if(x > 0) r[0] += trace;
     }
     else
-      cell_pencil<N, true, !LAST, 0>(s_tab, t64, FM, FC, FT, pv, qv, 0.0, 0.0, r, m, tl, tu);
+      cell_pencil<N, true, !LAST, 0>(s_tab, t64, FM, FC, FT, pv, qv, 0.0, 0.0, r, m, tl, tu, [](double &, double &) {});
     if(wf & kSpecial) special_faces<N>(a.sig + 3 * x, x > 0, x + 1 < n, own, qv[0], qv[N - 1], r[0], r[N - 1], tl, tu);
     auto store = [&](int64_t cell, int i, double v) {
       if constexpr(LAST)
@@ -381,8 +413,14 @@ struct OpXCfg
   static constexpr size_t smem() { return ((size_t)XT * TS + 2 * PENCILS + 2 * (size_t)N * CS + ROWS) * 8; }
 };
 
+constexpr int x_regs(int n)
+{
+  constexpr int r[9] = {0, 0, 40, 56, 56, 64, 72, 72, 72};
+  return r[n];
+}
+
 template<int DIM, int N>
-__global__ void __launch_bounds__(OpXCfg<DIM, N>::THREADS) op_x_kernel(OpLineArgs a)
+__global__ void __maxnreg__((x_regs(N))) op_x_kernel(OpLineArgs a)
 {
   using C = OpXCfg<DIM, N>;
   using T = OpTab<N>;
@@ -441,12 +479,16 @@ __global__ void __launch_bounds__(OpXCfg<DIM, N>::THREADS) op_x_kernel(OpLineArg
     const int FM = a.exps[3 * w], FC = a.exps[3 * w + 1], FT = a.exps[3 * w + 2];
     if(own)
     {
-      const double uL = x > 0 ? a.q[first(x - 1, g) + N * rr + N - 1] : negated(q[0]);
-      const double uR = x + 1 < nx ? a.q[first(x + 1, g) + N * rr] : negated(q[N - 1]);
-      cell_pencil<N, false, true, 1>(tab, t64, FM, FC, FT, q, q, uL, uR, r, m, tl, tu);
+      auto faces = [&](double &lo, double &hi) {
+        lo = x > 0 ? a.q[first(x - 1, g) + N * rr + N - 1] : negated(u[0]);
+        hi = x + 1 < nx ? a.q[first(x + 1, g) + N * rr] : negated(u[N - 1]);
+      };
+      double uL, uR;
+      faces(uL, uR);
+      cell_pencil<N, false, true, 1>(tab, t64, FM, FC, FT, q, q, uL, uR, r, m, tl, tu, faces);
     }
     else
-      cell_pencil<N, false, true, 0>(tab, t64, FM, FC, FT, q, q, 0.0, 0.0, r, m, tl, tu);
+      cell_pencil<N, false, true, 0>(tab, t64, FM, FC, FT, q, q, 0.0, 0.0, r, m, tl, tu, [](double &, double &) {});
     if(wf & kSpecial) special_faces<N>(a.sig + 3 * x, x > 0, x + 1 < nx, own, q[0], q[N - 1], r[0], r[N - 1], tl, tu);
     if(own)
 #pragma unroll
