@@ -26,8 +26,10 @@ void append_tables(std::vector<double> &buf)
     std::frexp(s * (1 + 1e-14L), &e);
     return 62 - e;
   };
+  // rows of nodes that are coarse ones have a single entry and are left out (transfer64.cuh)
+  constexpr int ROWS = T::ROWS;
   ext::Real row = 0, col = 0;
-  for(int r = 0; r < 2 * N; ++r)
+  for(int r = 1; r <= ROWS; ++r)
   {
     ext::Real s = 0;
     for(int m = 0; m < N; ++m) s += std::fabs(at(r, m));
@@ -36,23 +38,24 @@ void append_tables(std::vector<double> &buf)
   for(int m = 0; m < N; ++m)
   {
     ext::Real s = 0;
-    for(int r = 0; r < 2 * N; ++r) s += std::fabs(at(r, m));
+    for(int r = 1; r <= ROWS; ++r) s += std::fabs(at(r, m)) + std::fabs(at(2 * N - 1 - r, m));
     col = std::max(col, s);
   }
   const int32_t F[2] = {exponent(row), exponent(col)};
   std::vector<int64_t> t(T::SIZE + 1, 0);
-  for(int i = 0; i < N; ++i)
+  for(int i = 0; i < ROWS; ++i)
     for(int j = 0; j < T::HE; ++j)
     {
+      const ext::Real *e = E[1 + i];
       const bool mid = 2 * j == N - 1;
-      t[T::PE + i * T::LPE + j] = ext::limbs(mid ? at(i, j) : (at(i, j) + at(i, N - 1 - j)) / 2, F[0]);
-      if(!mid) t[T::PO + i * T::LPO + j] = ext::limbs((at(i, j) - at(i, N - 1 - j)) / 2, F[0]);
+      t[T::PE + i * T::LPE + j] = ext::limbs(mid ? e[j] : (e[j] + e[N - 1 - j]) / 2, F[0]);
+      if(!mid) t[T::PO + i * T::LPO + j] = ext::limbs((e[j] - e[N - 1 - j]) / 2, F[0]);
     }
   for(int i = 0; i < T::HE; ++i)
-    for(int j = 0; j < N; ++j)
+    for(int j = 0; j < ROWS; ++j)
     {
       // for the middle node both children's values have the same coefficient
-      const ext::Real a = at(j, i), b = at(2 * N - 1 - j, i);
+      const ext::Real a = at(1 + j, i), b = at(2 * N - 2 - j, i);
       t[T::RE + i * T::LR + j] = ext::limbs((a + b) / 2, F[1]);
       if(i < T::H) t[T::RO + i * T::LR + j] = ext::limbs((a - b) / 2, F[1]);
     }

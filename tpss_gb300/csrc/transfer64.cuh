@@ -4,17 +4,22 @@
 // N^2 products in even/odd form for all 2N results (and back). Prolongation widens the coarse cell
 // along x, y and z in turn (N^(d-1), 2 N^(d-1), 4 N^(d-1) pencils), restriction goes the other way. The
 // fine vector is read and written by the threads of the z (2D: y) pass, which hold a pencil of both children
-// each; their order runs through a child's layer, so that they read and write whole rows. Between
-// the passes the cell lives in shared memory as 64-bit integers with one exponent (fixed64.cuh):
-// every pass is scaled by 4, the room its coefficients' row sums leave, so its rounding is 2^-58 of the
-// cell's largest value.
-// Values the integers do not cover (infinities, NaN, magnitudes outside 2^(+-300)) take FP64 passes on the
-// same shared memory, cell by cell.
+// each; their order runs through a child's layer, so that they read and write whole rows.
 //
-// Measured, 16^3 coarse cells, k = 4 (4.1M fine values): prolongation 24.9 us, restriction 24.5 us, where the tree
+// Every pencil has a unit of its own, and between the passes the cell lives in shared memory in FP64. A fine
+// node that is a coarse one (the ends, and the middle for odd N) takes its value as it is in FP64, in both
+// directions: its row of the matrix has a single entry, and the others do not see it. The
+// remaining rows have no zeros, so that what sets a pencil's unit enters all of its results: one pass's rounding
+// is 2^-58 of the pencil's largest value, and small values next to large ones keep their digits.
+// Values the integers do not cover (infinities, NaN, magnitudes outside 2^(+-300)) take FP64 passes, pencil by
+// pencil.
+//
+// Measured, 16^3 coarse cells, k = 4 (4.1M fine values): prolongation 25 us, restriction 25.5 us, where the tree
 // of FP64 passes per child took 90 and 92 us (FP64 pipe). The fine values move in 10 and 5 us at the copy
 // rate; the rest is the serial chain of three passes, hidden behind the other CTAs of the SM only in
-// part. 2^3 coarse cells take 6 and 5 us instead of 25 and 27. Fetching the fine values that the prolongation adds to
+// part. 2^3 coarse cells take 5 us each way instead of 25 and 27. (One unit per cell, with the cell in
+// integers between the passes, took 25 and 26.5 us and lost a small value's digits next to a large one anywhere in
+// the cell.) Fetching the fine values that the prolongation adds to
 // before the passes instead of at the addition: 31.8 -> 24.9 us.
 #pragma once
 
@@ -29,14 +34,15 @@ template<int N>
 struct TrTab
 {
   static constexpr int pad2(int x) { return (x + 1) / 2 * 2; }
-  static constexpr int H = N / 2, HE = (N + 1) / 2;
-  static constexpr int LPE = pad2(HE), LPO = pad2(H), LR = pad2(N);
-  static constexpr int PE = 0;              // prolongation: N even rows (the first child's nodes)
-  static constexpr int PO = PE + N * LPE;   // N odd rows
-  static constexpr int RE = PO + N * LPO;   // restriction: HE even rows (the last one the middle node's)
-  static constexpr int RO = RE + HE * LR;   // H odd rows
+  static constexpr int H = N / 2, HE = (N + 1) / 2, ODD = N % 2;
+  static constexpr int ROWS = N - 1 - ODD;         // the first child's nodes 1 .. ROWS that are no coarse nodes
+  static constexpr int LPE = pad2(HE), LPO = pad2(H), LR = pad2(ROWS);
+  static constexpr int PE = 0;                     // prolongation: ROWS even rows
+  static constexpr int PO = PE + ROWS * LPE;       // ROWS odd rows
+  static constexpr int RE = PO + ROWS * LPO;       // restriction: HE even rows (the last one the middle node's)
+  static constexpr int RO = RE + HE * LR;          // H odd rows
   static constexpr int SIZE = RO + H * LR;
-  static constexpr int FEXP = 2 * N * N + SIZE;  // word with the two exponents F (int2)
+  static constexpr int FEXP = 2 * N * N + SIZE;    // word with the two exponents F (int2)
   static constexpr int WORDS = FEXP + 1;
 };
 
@@ -105,78 +111,135 @@ __device__ __forceinline__ int64_t dot4(const int2 *__restrict__ row, const int 
   return (S.value() << 2) + ((M.value() + (Q.value() >> 29)) >> 30);
 }
 
-// 2N results of both children from the N values get(m)
-template<int N, typename Get, typename Put>
-__device__ __forceinline__ void widen(const int2 *tab, const Get &get, const Put &put)
+// exponent of a pencil (1023: all zeros), -1: the integers do not cover it
+__device__ __forceinline__ int exponent(unsigned hi, unsigned lo)
+{
+  const int e = (int)(hi >> 20);
+  return (hi | lo) == 0 ? 1023 : e < 1023 - 300 || e > 1023 + 300 ? -1 : e;
+}
+__device__ __forceinline__ void magnitude(double v, unsigned &hi, unsigned &lo)
+{
+  hi = max(hi, (unsigned)__double2hiint(v) & 0x7fffffffu);
+  lo |= (unsigned)__double2loint(v);
+}
+
+// 2N results of both children, put(r, value), from a pencil's N values; E: FP64 rows. put_at is put for an r
+// that is not a constant
+template<int N, typename Put, typename PutAt>
+__device__ __forceinline__ void widen(const int2 *tab, const double *E, int F, const double (&v)[N], const Put &put,
+                                      const PutAt &put_at)
 {
   using T = TrTab<N>;
-  constexpr int H = T::H, HE = T::HE;
+  constexpr int H = T::H, HE = T::HE, ROWS = T::ROWS;
+  put(0, v[0]);
+  put(2 * N - 1, v[N - 1]);
+  if constexpr(T::ODD)
+  {
+    put(N - 1, v[H]);
+    put(N, v[H]);
+  }
+  if constexpr(N == 2)
+  {
+    // one value at the middle of both: exactly rounded in FP64, and no more work
+    const double s = fma(0.5, v[1], 0.5 * v[0]);
+    put(1, s);
+    put(2, s);
+    return;
+  }
+  unsigned hi = 0, lo = 0;
+#pragma unroll
+  for(int i = 0; i < N; ++i) magnitude(v[i], hi, lo);
+  const int e = exponent(hi, lo);
+  if(e < 0)
+  {
+    double w[N];  // (a copy, so that v stays in registers)
+#pragma unroll
+    for(int i = 0; i < N; ++i) w[i] = v[i];
+#pragma unroll 1
+    for(int r = 1; r < 2 * N - 1; ++r)
+    {
+      if(T::ODD && (r == N - 1 || r == N)) continue;
+      double s = 0.0;
+#pragma unroll 1
+      for(int m = 0; m < N; ++m) s = fma(E[r * N + m], w[m], s);
+      put_at(r, s);
+    }
+    return;
+  }
   int eh[HE], el[HE], oh[HE], ol[HE];
 #pragma unroll
   for(int j = 0; j < H; ++j)
   {
-    const int64_t a = get(j), b = get(N - 1 - j);
+    const int64_t a = fx::from_double(v[j], e), b = fx::from_double(v[N - 1 - j], e);
     fx::split(a + b, eh[j], el[j]);
     fx::split(a - b, oh[j], ol[j]);
   }
-  if constexpr(N % 2 == 1) fx::split(get(H), eh[H], el[H]);
+  if constexpr(T::ODD) fx::split(fx::from_double(v[H], e), eh[H], el[H]);
+  const int unit = e - 1023 - 58 + 62 - F;
 #pragma unroll
-  for(int i = 0; i < N; ++i)
+  for(int i = 0; i < ROWS; ++i)
   {
-    const int64_t e = dot4<HE>(tab + T::PE + i * T::LPE, eh, el), o = dot4<H>(tab + T::PO + i * T::LPO, oh, ol);
-    put(i, e + o);
-    put(2 * N - 1 - i, e - o);
+    const int64_t s = dot4<HE>(tab + T::PE + i * T::LPE, eh, el), o = dot4<H>(tab + T::PO + i * T::LPO, oh, ol);
+    put(1 + i, fx::to_double_alu(s + o, unit));
+    put(2 * N - 2 - i, fx::to_double_alu(s - o, unit));
   }
 }
 
-// N results from the 2N values get(m) of both children
-template<int N, typename Get, typename Put>
-__device__ __forceinline__ void narrow(const int2 *tab, const Get &get, const Put &put)
+// N results, put(m, value), from the 2N values of both children
+template<int N, typename Put>
+__device__ __forceinline__ void narrow(const int2 *tab, const double *E, int F, const double (&v)[2 * N], const Put &put)
 {
   using T = TrTab<N>;
-  constexpr int H = T::H;
-  int eh[N], el[N], oh[N], ol[N];
-#pragma unroll
-  for(int j = 0; j < N; ++j)
+  constexpr int H = T::H, ROWS = T::ROWS;
+  if constexpr(N == 2)
   {
-    const int64_t a = get(j), b = get(2 * N - 1 - j);
+    const double s = fma(0.5, v[2], 0.5 * v[1]);
+    put(0, v[0] + s);
+    put(1, v[3] + s);
+    return;
+  }
+  unsigned hi = 0, lo = 0;
+#pragma unroll
+  for(int j = 1; j <= ROWS; ++j)
+  {
+    magnitude(v[j], hi, lo);
+    magnitude(v[2 * N - 1 - j], hi, lo);
+  }
+  const int e = exponent(hi, lo);
+  if(e < 0)
+  {
+    double w[2 * N];
+#pragma unroll
+    for(int r = 0; r < 2 * N; ++r) w[r] = v[r];
+#pragma unroll 1
+    for(int i = 0; i < N; ++i)
+    {
+      double s = 0.0;
+#pragma unroll 1
+      for(int r = 0; r < 2 * N; ++r) s = fma(E[r * N + i], w[r], s);
+      put(i, s);
+    }
+    return;
+  }
+  int eh[ROWS + 1], el[ROWS + 1], oh[ROWS + 1], ol[ROWS + 1];
+#pragma unroll
+  for(int j = 0; j < ROWS; ++j)
+  {
+    const int64_t a = fx::from_double(v[1 + j], e), b = fx::from_double(v[2 * N - 2 - j], e);
     fx::split(a + b, eh[j], el[j]);
     fx::split(a - b, oh[j], ol[j]);
   }
-#pragma unroll(N <= 5 ? H : 1)
+  const int unit = e - 1023 - 58 + 62 - F;
+#pragma unroll
   for(int i = 0; i < H; ++i)
   {
-    const int64_t e = dot4<N>(tab + T::RE + i * T::LR, eh, el), o = dot4<N>(tab + T::RO + i * T::LR, oh, ol);
-    put(i, e + o);
-    put(N - 1 - i, e - o);
+    const int64_t s = dot4<ROWS>(tab + T::RE + i * T::LR, eh, el), o = dot4<ROWS>(tab + T::RO + i * T::LR, oh, ol);
+    const double lower = fx::to_double_alu(s + o, unit), upper = fx::to_double_alu(s - o, unit);
+    put(i, i == 0 ? v[0] + lower : lower);
+    put(N - 1 - i, i == 0 ? v[2 * N - 1] + upper : upper);
   }
-  if constexpr(N % 2 == 1) put(H, dot4<N>(tab + T::RE + H * T::LR, eh, el));
-}
-
-// the same in FP64, rolled
-template<int N, typename Get, typename Put>
-__device__ __forceinline__ void widen_fp64(const double *E, const Get &get, const Put &put)
-{
-#pragma unroll 1
-  for(int r = 0; r < 2 * N; ++r)
-  {
-    double v = 0.0;
-#pragma unroll 1
-    for(int m = 0; m < N; ++m) v = fma(E[r * N + m], get(m), v);
-    put(r, v);
-  }
-}
-template<int N, typename Get, typename Put>
-__device__ __forceinline__ void narrow_fp64(const double *E, const Get &get, const Put &put)
-{
-#pragma unroll 1
-  for(int i = 0; i < N; ++i)
-  {
-    double v = 0.0;
-#pragma unroll 1
-    for(int r = 0; r < 2 * N; ++r) v = fma(E[r * N + i], get(r), v);
-    put(i, v);
-  }
+  if constexpr(T::ODD)
+    put(H, v[N - 1] + v[N] + fx::to_double_alu(dot4<ROWS>(tab + T::RE + H * T::LR, eh, el), unit));
 }
 
 template<int DIM, int N, bool RESTRICT>
@@ -186,15 +249,14 @@ __global__ void __launch_bounds__(TrCfg<DIM, N>::THREADS) transfer64_kernel(TrAr
   using T = TrTab<N>;
   constexpr int ND = C::ND, PL = C::PL, PX = C::PX, SA = C::SA, F2 = 2 * N, L2 = N * N;
   __shared__ __align__(16) int2 s_tab[T::SIZE];
-  __shared__ int64_t s_a[C::CPB * C::A], s_b[C::CPB * C::B + 1];
-  __shared__ unsigned s_hi[C::CPB], s_lo[C::CPB];
+  __shared__ double s_a[C::CPB * C::A], s_b[C::CPB * C::B + 1];
   const int tid = threadIdx.x, slot = tid / PL, p = tid % PL;
   const int64_t cell = (int64_t)blockIdx.x * C::CPB + slot;
   const bool active = slot < C::CPB && cell < a.n_coarse;
   const int2 *src_tab = reinterpret_cast<const int2 *>(a.E + 2 * N * N);
   const int2 fexp = src_tab[T::SIZE];
+  const int F = RESTRICT ? fexp.y : fexp.x;
   for(int i = tid; i < T::SIZE; i += C::THREADS) s_tab[i] = src_tab[i];
-  if(tid < C::CPB) s_hi[tid] = s_lo[tid] = 0;
   // this thread's pencil of the last direction: node (X, Y) of the widened layer, in child (bx, by)
   const int bxy = p / (DIM == 2 ? N : L2), x = p % N, y = DIM == 2 ? 0 : p / N % N;
   const int bx = bxy % 2, by = bxy / 2, X = bx * N + x, Y = by * N + y;
@@ -204,101 +266,74 @@ __global__ void __launch_bounds__(TrCfg<DIM, N>::THREADS) transfer64_kernel(TrAr
   double *fine = a.fine + child * ND + (DIM == 2 ? x : x + N * y);
   const int64_t above = (DIM == 2 ? nf0 : nf0 * nf1) * ND;  // the upper child
   double *coarse = a.coarse + cell * ND;
-  int64_t *A = s_a + (slot < C::CPB ? slot : 0) * C::A, *B = s_b + (slot < C::CPB ? slot : 0) * C::B;
-  double *Ad = reinterpret_cast<double *>(A), *Bd = reinterpret_cast<double *>(B);
+  double *A = s_a + (slot < C::CPB ? slot : 0) * C::A, *B = s_b + (slot < C::CPB ? slot : 0) * C::B;
   auto fine_at = [&](int r) -> double & { return fine[(r >= N ? above : 0) + (r >= N ? r - N : r) * (DIM == 2 ? N : L2)]; };
+  // pencil q along y (3D: of the arrays between the x and the z pass)
+  auto ay = [&](int q, int j) { return (q / F2 * N + j) * SA + q % F2; };
+  auto by_ = [&](int q, int j) { return (q / F2 * F2 + j) * F2 + q % F2; };
+  // pencil along the last direction
+  auto last = [&](int j) { return DIM == 2 ? j * SA + X : (j * F2 + Y) * F2 + X; };
   __syncthreads();
-  // the values of this thread's first pass and the cell's largest exponent
-  constexpr int NV = RESTRICT ? 2 * N : N;
-  const bool first = active && (RESTRICT || p < PX);
-  double v[NV], f[RESTRICT ? 1 : 2 * N];  // f: what the prolongation adds to, on its way during the passes
-  unsigned hi = 0, lo = 0;
   if constexpr(!RESTRICT)
+  {
+    double f[2 * N], v[N];  // f: what the prolongation adds to, on its way during the passes
     if(active)
     {
 #pragma unroll
       for(int r = 0; r < 2 * N; ++r) f[r] = fine_at(r);
     }
-  if(first)
-  {
+    if(active && p < PX)
+    {
 #pragma unroll
-    for(int i = 0; i < NV; ++i)
-    {
-      v[i] = RESTRICT ? fine_at(i) : coarse[p * N + i];
-      hi = max(hi, (unsigned)__double2hiint(v[i]) & 0x7fffffffu);
-      lo |= (unsigned)__double2loint(v[i]);
-    }
-    atomicMax(s_hi + slot, hi);
-    if(lo) atomicOr(s_lo + slot, lo);
-  }
-  __syncthreads();
-  if(active)
-  {
-    hi = s_hi[slot];
-    lo = s_lo[slot];
-  }
-  const int ex = (int)(hi >> 20);
-  const bool slow = active && (ex < 1023 - 300 || ex > 1023 + 300) && (hi | lo) != 0;
-  const int emax = hi == 0 ? 1023 : ex;
-  auto value = [&](int i) { return fx::from_double(v[i], emax); };
-  const int unit = emax - 1023 - 58 + DIM * (62 - (RESTRICT ? fexp.y : fexp.x));  // exponent of the results
-  // pencil q along y (3D: of the arrays between the x and the z pass)
-  auto ay = [&](int q, int j) { return (q / F2 * N + j) * SA + q % F2; };
-  auto by_ = [&](int q, int j) { return (q / F2 * F2 + j) * F2 + q % F2; };
-  if constexpr(!RESTRICT)
-  {
-    if(first)
-    {
-      if(!slow) widen<N>(s_tab, value, [&](int r, int64_t w) { A[p * SA + r] = w; });
-      else widen_fp64<N>(a.E, [&](int i) { return coarse[p * N + i]; }, [&](int r, double w) { Ad[p * SA + r] = w; });
+      for(int i = 0; i < N; ++i) v[i] = coarse[p * N + i];
+      auto put = [&](int r, double w) { A[p * SA + r] = w; };
+      widen<N>(s_tab, a.E, F, v, put, put);
     }
     __syncthreads();
     if constexpr(DIM == 3)
     {
       if(active && p < F2 * N)
       {
-        if(!slow) widen<N>(s_tab, [&](int j) { return A[ay(p, j)]; }, [&](int r, int64_t w) { B[by_(p, r)] = w; });
-        else widen_fp64<N>(a.E, [&](int j) { return Ad[ay(p, j)]; }, [&](int r, double w) { Bd[by_(p, r)] = w; });
+#pragma unroll
+        for(int j = 0; j < N; ++j) v[j] = A[ay(p, j)];
+        auto put = [&](int r, double w) { B[by_(p, r)] = w; };
+        widen<N>(s_tab, a.E, F, v, put, put);
       }
       __syncthreads();
     }
     if(active)
     {
-      // pencil along the last direction
-      auto in = [&](int j) { return DIM == 2 ? j * SA + X : (j * F2 + Y) * F2 + X; };
-      if(!slow)
-        widen<N>(s_tab, [&](int j) { return (DIM == 2 ? A : B)[in(j)]; },
-                 [&](int r, int64_t w) { fine_at(r) = f[r] + fx::to_double_alu(w, unit); });
-      else
-        widen_fp64<N>(a.E, [&](int j) { return (DIM == 2 ? Ad : Bd)[in(j)]; }, [&](int r, double w) { fine_at(r) += w; });
+#pragma unroll
+      for(int j = 0; j < N; ++j) v[j] = (DIM == 2 ? A : B)[last(j)];
+      widen<N>(s_tab, a.E, F, v, [&](int r, double w) { fine_at(r) = f[r] + w; },
+               [&](int r, double w) { fine_at(r) += w; });
     }
   }
   else
   {
+    double v[2 * N];
     if(active)
     {
-      auto out = [&](int j) { return DIM == 2 ? j * SA + X : (j * F2 + Y) * F2 + X; };
-      if(!slow) narrow<N>(s_tab, value, [&](int j, int64_t w) { (DIM == 2 ? A : B)[out(j)] = w; });
-      else
-        narrow_fp64<N>(a.E, [&](int r) { return fine_at(r); }, [&](int j, double w) { (DIM == 2 ? Ad : Bd)[out(j)] = w; });
+#pragma unroll
+      for(int r = 0; r < 2 * N; ++r) v[r] = fine_at(r);
+      narrow<N>(s_tab, a.E, F, v, [&](int j, double w) { (DIM == 2 ? A : B)[last(j)] = w; });
     }
     __syncthreads();
     if constexpr(DIM == 3)
     {
       if(active && p < F2 * N)
       {
-        if(!slow) narrow<N>(s_tab, [&](int r) { return B[by_(p, r)]; }, [&](int j, int64_t w) { A[ay(p, j)] = w; });
-        else narrow_fp64<N>(a.E, [&](int r) { return Bd[by_(p, r)]; }, [&](int j, double w) { Ad[ay(p, j)] = w; });
+#pragma unroll
+        for(int r = 0; r < 2 * N; ++r) v[r] = B[by_(p, r)];
+        narrow<N>(s_tab, a.E, F, v, [&](int j, double w) { A[ay(p, j)] = w; });
       }
       __syncthreads();
     }
     if(active && p < PX)
     {
-      if(!slow)
-        narrow<N>(s_tab, [&](int r) { return A[p * SA + r]; },
-                  [&](int i, int64_t w) { coarse[p * N + i] += fx::to_double(w, unit); });
-      else
-        narrow_fp64<N>(a.E, [&](int r) { return Ad[p * SA + r]; }, [&](int i, double w) { coarse[p * N + i] += w; });
+#pragma unroll
+      for(int r = 0; r < 2 * N; ++r) v[r] = A[p * SA + r];
+      narrow<N>(s_tab, a.E, F, v, [&](int i, double w) { coarse[p * N + i] += w; });
     }
   }
 }
