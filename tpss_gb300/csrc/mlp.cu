@@ -410,7 +410,11 @@ double mlp_loss_only(tpss_mlp &m, const float *x, const float *target, int64_t r
 void mlp_infer(const tpss_mlp &mc, const float *x_dev, int64_t rows, float *y_dev, cudaStream_t s)
 {
   tpss_mlp &m = const_cast<tpss_mlp &>(mc);  // activation scratch only
-  mlp_forward(m, x_dev, rows, s, y_dev);
+  // y may be x: the last of several layers reads activations, a single one x itself
+  const bool single = m.n_layers() == 1;
+  mlp_forward(m, x_dev, rows, s, single ? nullptr : y_dev);
+  if(single)
+    TPSS_CUDA(cudaMemcpyAsync(y_dev, m.act[0].ptr, sizeof(float) * rows * m.n_out, cudaMemcpyDeviceToDevice, s));
 }
 
 int mlp_n_in(const tpss_mlp &m) { return m.n_in; }
