@@ -292,8 +292,10 @@ void launch_gemm(const GemmArgs &g, cudaStream_t s)
   TPSS_CUDA(cudaGetLastError());
 }
 
-// weight and bias gradient of one layer; the rows are cut into chunks until the tiles fill the chip
-// twice, but not below 64 rows
+// weight and bias gradient of one layer; the rows are cut into chunks until the tiles fill the chip's 152 SMs
+// twice, but not below 64 rows. The count is fixed, so that the order of the sums depends on the sizes alone
+constexpr int kWgradCtas = 304;
+
 void launch_wgrad(tpss_mlp &m, const float *delta, const float *x, int64_t rows, int ni, int no, float *dW, float *db,
                   cudaStream_t s)
 {
@@ -308,7 +310,7 @@ void launch_wgrad(tpss_mlp &m, const float *delta, const float *x, int64_t rows,
   const bool large = rows >= 4096;
   const int T = large ? 64 : 32;
   const int64_t tiles = ((g.M + T - 1) / T) * ((g.N + T - 1) / T);
-  int64_t chunks = std::min<int64_t>((2 * num_sms() + tiles - 1) / tiles, (rows + 63) / 64);
+  int64_t chunks = std::min<int64_t>((kWgradCtas + tiles - 1) / tiles, (rows + 63) / 64);
   g.chunk = (rows + chunks - 1) / chunks;
   chunks = (rows + g.chunk - 1) / g.chunk;
   g.db = db;
