@@ -15,7 +15,10 @@
  *  - Work is ordered on the caller's stream (a cudaStream_t passed as void*; NULL = legacy
  *    default stream).  Handles are not reentrant: one stream at a time per handle, as the
  *    reference's SchwarzPreconditioner::vmult is const but mutates timers and scratch
- *    (schwarz_preconditioner.h:184-236).
+ *    (schwarz_preconditioner.h:184-236).  That includes tpss_operator_vmult and the FP64
+ *    smoother, which keep intermediate vectors in their handle.  Their calls on two streams
+ *    run one after the other; a call that a CUDA graph has captured is not ordered with calls
+ *    outside the graph, nor with the same graph's other branches: do not replay it beside them.
  *  - No torch or deal.II types appear here; plain pointers and sizes only.
  */
 #ifndef TPSS_GPU_H
@@ -136,7 +139,10 @@ int tpss_operator_create(const tpss_layout *layout, double ip_factor, tpss_opera
 /* The same with a TPSS_PENALTY_* mode (tpss_operator_create uses TPSS_PENALTY_REFERENCE). */
 int tpss_operator_create_penalty(const tpss_layout *layout, double ip_factor, int penalty_mode,
                                  tpss_operator **out);
-/* MF::Operator::vmult (apps/laplace_integrator.h:578-598), FP64. */
+/* MF::Operator::vmult (apps/laplace_integrator.h:578-598), FP64.  On Cartesian levels but the
+ * smallest the operator holds intermediate vectors for it, 4 values per DoF in 3D and 2 in 2D, allocated
+ * when it is created; without room for them then it uses a kernel that needs none (3D DGQ4:
+ * 3.3 times the time).  A product allocates nothing. */
 int tpss_operator_vmult(tpss_operator *op, double *dst, const double *src, void *stream);
 /* The same product in FP32 arithmetic on FP64 vectors (src is converted once into a scratch
  * copy owned by the operator; dst is written in FP64): the level operator of a single-precision
@@ -194,7 +200,10 @@ int tpss_precond_create(const tpss_layout *layout, tpss_operator *op,
 int tpss_precond_create_shallow(const tpss_precond *other, const tpss_precond_desc *desc,
                                 tpss_precond **out);
 /* SchwarzPreconditioner::vmult (schwarz_preconditioner.templates.h:209-239): dst is set to
- * zero and receives sum over colors of omega R_j^T A_j^-1 R_j src. */
+ * zero and receives sum over colors of omega R_j^T A_j^-1 R_j src.  FP64, additive vertex patches on a
+ * Cartesian level: the handle (a shallow copy too) holds intermediate vectors, 10 values per DoF
+ * in 3D and 4 in 2D, allocated when it is created; without room for them then it applies the
+ * patches color by color (1.7 times the time).  These applications allocate nothing. */
 int tpss_precond_vmult(tpss_precond *p, double *dst, const double *src, void *stream);
 /* vmult_add (schwarz_preconditioner.templates.h:185-194): dst += P src. */
 int tpss_precond_vmult_add(tpss_precond *p, double *dst, const double *src, void *stream);
@@ -211,7 +220,7 @@ int tpss_precond_Tvmult(tpss_precond *p, double *dst, const double *src, void *s
  * has started: a host application that owns all device memory through its own pool and
  * forbids library-side cudaMalloc/cudaFree after setup, or one that cannot afford the device
  * synchronization of cudaFree or an out-of-memory failure in the middle of an iteration.
- * (tpss_precond_vmult grows its scratch buffer with cudaMalloc on first use.)
+ * (For this smoother tpss_precond_vmult grows its scratch buffer with cudaMalloc on first use.)
  *
  * The scratch for the partial sums of cells shared between work items is a fixed device array
  * of 32 MiB (8 Mi floats), held by every GPU that loads the library until the process exits.

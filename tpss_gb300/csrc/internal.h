@@ -73,9 +73,13 @@ int guarded(F &&f)
 struct ScratchOrder
 {
   std::mutex m;
-  cudaEvent_t ev = nullptr;
+  cudaEvent_t ev = nullptr;  // created with the scratch, as its handle is
   ScratchOrder() = default;
   ScratchOrder(const ScratchOrder &) = delete;
+  void create()
+  {
+    if(!ev) TPSS_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+  }
   ~ScratchOrder()
   {
     if(ev) cudaEventDestroy(ev);
@@ -95,16 +99,13 @@ public:
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     TPSS_CUDA(cudaStreamIsCapturing(s, &cs));
     capturing = cs != cudaStreamCaptureStatusNone;
-    if(capturing) return;
-    if(o.ev) TPSS_CUDA(cudaStreamWaitEvent(s, o.ev, 0));
-    else TPSS_CUDA(cudaEventCreateWithFlags(&o.ev, cudaEventDisableTiming));
+    if(!capturing) TPSS_CUDA(cudaStreamWaitEvent(s, o.ev, 0));
   }
   ScratchUse(const ScratchUse &) = delete;
   ~ScratchUse()
   {
     if(!capturing) cudaEventRecord(o.ev, s);
   }
-  bool may_allocate() const { return !capturing; }
 };
 
 // device buffer with RAII
@@ -143,6 +144,23 @@ struct DeviceBuffer
       TPSS_CUDA(cudaMalloc(&ptr, count * sizeof(T)));
       n = count;
     }
+  }
+  // false (and empty) when the device has no room; any other error is thrown
+  bool try_resize(size_t count)
+  {
+    release();
+    if(!count) return true;
+    T *p = nullptr;
+    const cudaError_t e = cudaMalloc(&p, count * sizeof(T));
+    if(e == cudaErrorMemoryAllocation)
+    {
+      cudaGetLastError();
+      return false;
+    }
+    TPSS_CUDA(e);
+    ptr = p;
+    n = count;
+    return true;
   }
   void upload(const T *host, size_t count)
   {
@@ -266,11 +284,12 @@ struct MappedOperator
 namespace tpss
 {
 // line-by-line FP64 operator (sipg_lines.cu): tables of all directions in one buffer, and the
-// intermediate vectors (4 per level in 3D, 2 in 2D)
+// intermediate vectors (4 per level in 3D, 2 in 2D). Both empty where the cell-wise kernel is faster and where the
+// device had no room for them when the operator was created
 struct OpLines
 {
   DeviceBuffer<int64_t> tables;
-  size_t off_tab[3] = {}, off_tab64[3] = {}, off_sig[3] = {}, off_exps[3] = {}, off_width[3] = {};
+  size_t off_tab = 0, off_tab64 = 0, off_exps = 0, off_sig[3] = {}, off_width[3] = {};
   DeviceBuffer<double> buf;
   ScratchOrder order;
 };
@@ -401,7 +420,8 @@ struct tpss_precond
   tpss_precond_desc desc{};
   tpss::DeviceBuffer<double> residual;  // multiplicative scratch
   tpss::DeviceBuffer<int> flag;         // finiteness check
-  tpss::DeviceBuffer<double> sweep[3];  // direction-by-direction smoother: line arrays (sweep64.cuh)
+  tpss::DeviceBuffer<double> sweep;     // direction-by-direction smoother: line arrays (sweep64.cuh), empty where
+                                        // it does not apply or the device had no room at creation
   tpss::ScratchOrder sweep_order;
   tpss::DeviceBuffer<float> halo;       // streamed kernel: partial sums of shared cells
   tpss::DeviceBuffer<int64_t> fix_rec[8];  // streamed kernel: shared-cell list per variant
@@ -502,8 +522,7 @@ void extract_local_matrices(const tpss_layout &L, const tpss_operator &op, int64
 // cellwise: sipg_kernel also where the line-by-line form applies, with the rounding it has
 void operator_apply(tpss_operator *op, double *dst, const double *src, cudaStream_t s,
                     const double *rhs = nullptr, bool cellwise = false);
-// line-by-line form of the FP64 product on a Cartesian level; false without tables or room for its
-// intermediate vectors (also while a stream is captured before the first product)
+// line-by-line form of the FP64 product on a Cartesian level, set up with the operator; false without it
 void build_op_lines(tpss_operator &op, const tpss_layout &L, Penalty pen);
 bool op_lines_apply(tpss_operator &op, double *dst, const double *src, cudaStream_t s, const double *rhs);
 // the same operator in FP32 arithmetic (FP64 vectors; the source is converted once into a

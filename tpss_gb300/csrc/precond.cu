@@ -13,7 +13,6 @@
 #include <chrono>
 #include <cmath>
 #include <cstring>
-#include <optional>
 
 #include "internal.h"
 
@@ -801,27 +800,14 @@ std::array<size_t, 3> sweep_sizes(const tpss_layout &L)
   return {mx * gy * gz, mx * my * gz, mx * my * gz};
 }
 
-// Holds the line arrays, or gets them if it may: not inside a stream capture, and not when the device
-// has no room for them (the per-color kernel then does without).
-bool sweep_scratch(tpss_precond *p, bool may_allocate)
+// Line arrays of a new handle, where the sweep applies and the device has room for them (the per-color
+// kernel does without): decided here once, so that every application takes the same route, also inside a
+// stream capture.
+void allocate_sweep(tpss_precond *p)
 {
+  if(!sweep_eligible(p)) return;
   const auto n = sweep_sizes(*p->tables->layout);
-  bool have = true;
-  for(int i = 0; i < 3; ++i) have = have && p->sweep[i].n >= n[i];
-  if(have) return true;
-  if(!may_allocate) return false;
-  try
-  {
-    for(int i = 0; i < 3; ++i)
-      if(p->sweep[i].n < n[i]) p->sweep[i].resize(n[i]);
-  }
-  catch(const Error &e)
-  {
-    cudaGetLastError();
-    for(auto &b : p->sweep) b.release();
-    return false;
-  }
-  return true;
+  if(p->sweep.try_resize(n[0] + n[1] + n[2])) p->sweep_order.create();
 }
 
 void launch_sweep(tpss_precond *p, double *dst, const double *src, cudaStream_t s)
@@ -831,9 +817,10 @@ void launch_sweep(tpss_precond *p, double *dst, const double *src, cudaStream_t 
   l.tables = p->tables.get();
   l.src = src;
   l.dst = dst;
-  l.a = p->sweep[0].ptr;
-  l.b = p->sweep[1].ptr;
-  l.c = p->sweep[2].ptr;
+  const auto n = sweep_sizes(*l.layout);
+  l.a = p->sweep.ptr;
+  l.b = l.a + n[0];
+  l.c = l.b + n[1];
   l.omega = p->desc.relaxation;
   l.ras = p->desc.use_ras_weights != 0;
   const int part = l.layout->k % 3;
@@ -891,10 +878,7 @@ void precond_vmult(tpss_precond *p, double *dst, const double *src, cudaStream_t
   TPSS_REQUIRE(dst && src, "null vector");
   TPSS_REQUIRE(dst != src, "dst and src must not alias");
   ScopedTimer step(p, 4, s);
-  std::optional<ScratchUse> use;
-  if(sweep_eligible(p)) use.emplace(p->sweep_order, s);
-  const bool sweep = use && sweep_scratch(p, use->may_allocate());
-  if(!sweep) use.reset();
+  const bool sweep = p->sweep.n > 0;
   if(!sweep && !(L.smoother_variant == TPSS_ADDITIVE && use_stream(p)))
     TPSS_CUDA(cudaMemsetAsync(dst, 0, sizeof(double) * L.n_dofs, s));
   if(L.smoother_variant == TPSS_ADDITIVE)
@@ -902,8 +886,8 @@ void precond_vmult(tpss_precond *p, double *dst, const double *src, cudaStream_t
     ScopedTimer t(p, 1, s);
     if(sweep)
     {
+      const ScratchUse use(p->sweep_order, s);
       launch_sweep(p, dst, src, s);  // writes every cell of dst
-      use.reset();
     }
     else if(use_stream(p))
     {
@@ -988,7 +972,7 @@ extern "C" int tpss_precond_create(const tpss_layout *layout, tpss_operator *op,
     p->tables = build_local_solvers(*layout, op, *desc);
     if(desc->use_ras_boolean_weights) build_keep_tables(*layout, *p->tables);
     if(desc->precision == TPSS_FP64) build_fixed_tables(*p->tables);
-    if(sweep_eligible(p.get())) sweep_scratch(p.get(), true);
+    allocate_sweep(p.get());
     p->timers.resize(5);
     for(int i = 0; i < 5; ++i) p->timers[i].name = kTimerNames[i];
     p->timers[2].time = p->tables->setup_seconds;
@@ -1022,6 +1006,7 @@ extern "C" int tpss_precond_create_shallow(const tpss_precond *other, const tpss
     validate_ras_boolean(*p->tables->layout, *desc);
     if(desc->use_ras_boolean_weights) build_keep_tables(*p->tables->layout, *p->tables);
     if(desc->precision == TPSS_FP64) build_fixed_tables(*p->tables);
+    allocate_sweep(p.get());
     p->timers = other->timers;
     *out = p.release();
   });
@@ -1163,7 +1148,7 @@ extern "C" int tpss_precond_autotune(tpss_precond *p, double *dst, const double 
     // (dense local inverses have a single kernel)
     const bool streamed = use_stream(p);
     const int nv = streamed ? stream_variant_count(L)
-                   : p->tables->dense || (sweep_eligible(p) && sweep_scratch(p, true)) ? 1
+                   : p->tables->dense || p->sweep.n ? 1
                                       : fd_variants(p->desc.precision == TPSS_FP32, L.dim, L.k, L.ncp);
     int &variant = streamed ? p->stream_variant : p->color_variant;
     if(n_variants) *n_variants = nv;

@@ -83,20 +83,26 @@ template<int N>
 void build(tpss_operator &op, const tpss_layout &L, Penalty pen)
 {
   using T = OpTab<N>;
-  const ext::Element<N> s(make_shape_1d(L.k));
+  static const ext::Element<N> s(make_shape_1d(N - 1));  // (0.1 ms and more in the 113 bits of an Arm host)
   const double gamma = double(L.k) * (L.k + 1);
   OpLines &O = op.lines;
-  // per direction: [integer tables][FP64 tables][sigma: 3 per cell][exponents: 3 per width][width per cell]
-  std::vector<int64_t> buf;
+  // of all directions' distinct widths: [integer tables][FP64 tables][exponents: 3 per width]; per direction:
+  // [sigma: 3 per cell][width per cell]
+  std::vector<int64_t> buf, ti;
+  std::map<double, int> id;
+  std::vector<double> t64;
+  std::vector<int> exps;
+  auto put = [&](const void *p, size_t words) {
+    const size_t at = buf.size();
+    buf.resize(at + words);
+    std::memcpy(buf.data() + at, p, words * 8);
+    return at;
+  };
   for(int d = 0; d < L.dim; ++d)
   {
     const int n = L.nc[d];
     const double *h = L.h[d].data();
-    std::map<double, int> id;
     std::vector<int32_t> width(n + n % 2, 0);
-    std::vector<double> t64;
-    std::vector<int> exps;
-    std::vector<int64_t> ti;
     for(int c = 0; c < n; ++c)
     {
       auto it = id.find(h[c]);
@@ -126,20 +132,14 @@ void build(tpss_operator &op, const tpss_layout &L, Penalty pen)
       sig[3 * c + 2] = pen.in * gamma / h[c];
       if(c == 0 || c == n - 1 || h[c - 1] != h[c] || h[c + 1] != h[c]) width[c] |= kSpecial;
     }
-    if(exps.size() % 2) exps.push_back(0);
-    auto put = [&](const void *p, size_t words) {
-      const size_t at = buf.size();
-      buf.resize(at + words);
-      std::memcpy(buf.data() + at, p, words * 8);
-      return at;
-    };
-    if(buf.size() % 2) buf.push_back(0);  // table rows are read as 16-byte pairs
-    O.off_tab[d] = put(ti.data(), ti.size());
-    O.off_tab64[d] = put(t64.data(), t64.size());
     O.off_sig[d] = put(sig.data(), sig.size());
-    O.off_exps[d] = put(exps.data(), exps.size() / 2);
     O.off_width[d] = put(width.data(), width.size() / 2);
   }
+  if(exps.size() % 2) exps.push_back(0);
+  O.off_exps = put(exps.data(), exps.size() / 2);
+  O.off_tab64 = put(t64.data(), t64.size());
+  if(buf.size() % 2) buf.push_back(0);  // table rows are read as 16-byte pairs
+  O.off_tab = put(ti.data(), ti.size());
   O.tables.upload(buf.data(), buf.size());
 }
 
@@ -152,10 +152,10 @@ void run(const tpss_operator &op, double *buf, double *dst, const double *src, c
   auto args = [&](int d) {
     OpLineArgs a{};
     const int64_t *b = O.tables.ptr;
-    a.tab = reinterpret_cast<const int2 *>(b + O.off_tab[d]);
-    a.tab64 = reinterpret_cast<const double *>(b + O.off_tab64[d]);
+    a.tab = reinterpret_cast<const int2 *>(b + O.off_tab);
+    a.tab64 = reinterpret_cast<const double *>(b + O.off_tab64);
     a.sig = reinterpret_cast<const double *>(b + O.off_sig[d]);
-    a.exps = reinterpret_cast<const int *>(b + O.off_exps[d]);
+    a.exps = reinterpret_cast<const int *>(b + O.off_exps);
     a.width = reinterpret_cast<const int32_t *>(b + O.off_width[d]);
     a.cell_start = L.lexicographic ? nullptr : L.d_cell_start.ptr;
     for(int e = 0; e < 3; ++e) a.nc[e] = L.nc[e];
@@ -231,17 +231,12 @@ void for_size(int np, const F &f)
 }
 }  // namespace
 
-void build_op_lines(tpss_operator &op, const tpss_layout &L, Penalty pen)
-{
-  for_size(L.np, [&](auto n) { build<decltype(n)::value>(op, L, pen); });
-}
-
 // Whether the passes are faster than the cell-wise kernel. On small levels both are latency: the passes take 12.4
 // (2D) and 18.6 us (3D) whatever the degree, the cell-wise kernel 9, 11.5 and 14.5 us for k = 1, 2, 3 in 2D and
 // 10.4, 13.8, 14.8, 18 and 21 us for k = 1 .. 5 in 3D; beyond that its multiply-adds cost 1.7 us per million
 // (2 per clock and SM), the passes' about 0.28 of that. The lines below are where the two meet
 // (measured equal: 2D k = 1 160^2 cells, 14.4 and 14.5 us; 3D k = 4 6^3, 18.6 and 19.1)
-bool lines_pay(const tpss_layout &L)
+static bool lines_pay(const tpss_layout &L)
 {
   static const double from[2][8] = {{0, 4.6, 1.4, 0, 0, 0, 0, 0}, {0, 11.3, 7.8, 4.3, 0.8, 0, 0, 0}};
   const double n = L.np, cells = (double)L.nc[0] * L.nc[1] * (L.dim == 3 ? L.nc[2] : 1);
@@ -249,28 +244,23 @@ bool lines_pay(const tpss_layout &L)
   return cells * fma * 1.7e-6 >= from[L.dim - 2][L.k];
 }
 
-// false: where the cell-wise kernel is faster, not inside a stream capture before a first call outside it, and not when the device has no room
-// for the intermediate vectors (the cell-wise kernel then does without)
+// Tables and intermediate vectors, allocated with the operator: a first product costs what the others do, and one
+// inside a stream capture takes the same route. Whether there is room is decided here once.
+void build_op_lines(tpss_operator &op, const tpss_layout &L, Penalty pen)
+{
+  if(!lines_pay(L)) return;
+  OpLines &O = op.lines;
+  if(!O.buf.try_resize((size_t)L.n_dofs * (L.dim == 3 ? 4 : 2))) return;
+  O.order.create();
+  for_size(L.np, [&](auto n) { build<decltype(n)::value>(op, L, pen); });
+}
+
 bool op_lines_apply(tpss_operator &op, double *dst, const double *src, cudaStream_t s, const double *rhs)
 {
   const tpss_layout &L = *op.layout;
   OpLines &O = op.lines;
-  if(O.tables.n == 0 || !lines_pay(L)) return false;
-  const size_t need = (size_t)L.n_dofs * (L.dim == 3 ? 4 : 2);
+  if(O.buf.n == 0) return false;
   const ScratchUse use(O.order, s);
-  if(O.buf.n < need)
-  {
-    if(!use.may_allocate()) return false;
-    try
-    {
-      O.buf.resize(need);
-    }
-    catch(const Error &)
-    {
-      cudaGetLastError();
-      return false;
-    }
-  }
   for_size(L.np, [&](auto n) {
     if(L.dim == 2) run<2, decltype(n)::value>(op, O.buf.ptr, dst, src, s, rhs);
     else run<3, decltype(n)::value>(op, O.buf.ptr, dst, src, s, rhs);
