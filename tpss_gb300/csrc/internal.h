@@ -522,6 +522,8 @@ void extract_local_matrices(const tpss_layout &L, const tpss_operator &op, int64
 // cellwise: sipg_kernel also where the line-by-line form applies, with the rounding it has
 void operator_apply(tpss_operator *op, double *dst, const double *src, cudaStream_t s,
                     const double *rhs = nullptr, bool cellwise = false);
+// tpss_operator_create_penalty; lines: with the line-by-line form
+int operator_create(const tpss_layout *layout, double ip_factor, int penalty_mode, bool lines, tpss_operator **out);
 // line-by-line form of the FP64 product on a Cartesian level, set up with the operator; false without it
 void build_op_lines(tpss_operator &op, const tpss_layout &L, Penalty pen);
 bool op_lines_apply(tpss_operator &op, double *dst, const double *src, cudaStream_t s, const double *rhs);

@@ -262,8 +262,8 @@ struct tpss_mg
   // in the last bit of a value at a rounding border becomes 6e-8 of it, and on a coarse level that spreads
   // over the domain: with the line-by-line operator and the integer transfers, two of six 32^3 V-cycles
   // (k = 4) came out 3e-11 and 1e-9 away from those with the cell-wise ones, no more and no less accurate.
-  // Such a V-cycle keeps the cell-wise kernels and with them its results to the bit (2.60 ms instead of
-  // 1.69); with FP64 smoothers the two agree to 1e-13.
+  // Such a hierarchy keeps the cell-wise kernels and with them its results to the bit (2.60 ms instead of
+  // 1.69): its operators have no line-by-line form. With FP64 smoothers the two agree to 1e-13.
   bool fp32_levels = false;
   ~tpss_mg()
   {
@@ -293,7 +293,7 @@ void level_residual_op(tpss_mg *mg, MgLevel &c, cudaStream_t s)
   if(mg->desc.vcycle_precision == TPSS_FP32)
     operator_apply_f32(c.op, c.t.ptr, c.x.ptr, s, c.b.ptr);
   else
-    operator_apply(c.op, c.t.ptr, c.x.ptr, s, c.b.ptr, mg->fp32_levels);
+    operator_apply(c.op, c.t.ptr, c.x.ptr, s, c.b.ptr);
 }
 
 TransferArith transfer_arith(const tpss_mg *mg)
@@ -356,7 +356,7 @@ void coarse_cg(tpss_mg *mg, cudaStream_t s)
   {
     for(it = 1; it <= n; ++it)
     {
-      operator_apply(c.op, Ap, p, s, nullptr, mg->fp32_levels);
+      operator_apply(c.op, Ap, p, s);
       vec_dot(n, p, Ap, mg->partial.ptr, pAp, s);
       cg_update_xr<<<grid_for(n), 256, 0, s>>>(n, x, r, p, Ap, rz, pAp);
       vec_dot(n, r, r, mg->partial.ptr, rz_new, s);
@@ -550,6 +550,8 @@ extern "C" int tpss_mg_create(const tpss_mg_desc *d, tpss_mg **out)
     auto mg = std::make_unique<tpss_mg>();
     mg->desc = *d;
     mg->lv.resize(nl);
+    auto level_precision = [&](int l) { return (d->fp64_level_mask >> l) & 1 ? (int)TPSS_FP64 : (int)d->precision; };
+    for(int l = 1; l < nl; ++l) mg->fp32_levels = mg->fp32_levels || level_precision(l) == TPSS_FP32;
     std::vector<double> coords;
     for(int l = 0; l < nl; ++l)
     {
@@ -581,18 +583,17 @@ extern "C" int tpss_mg_create(const tpss_mg_desc *d, tpss_mg **out)
       for(int dd = 0; dd < 3; ++dd) ld.n_cells[dd] = dd < d->dim ? (d->n_rep << l) : 1;
       int rc = tpss_layout_create(&ld, &lv.L);
       if(rc) fail(rc, tpss_last_error());
-      rc = tpss_operator_create_penalty(lv.L, d->ip_factor, d->penalty_mode, &lv.op);
+      rc = operator_create(lv.L, d->ip_factor, d->penalty_mode, !mg->fp32_levels, &lv.op);
       if(rc) fail(rc, tpss_last_error());
       if(l > 0)
       {
         tpss_precond_desc pd{};
         pd.relaxation = d->relaxation;
-        pd.precision = (d->fp64_level_mask >> l) & 1 ? TPSS_FP64 : d->precision;
+        pd.precision = level_precision(l);
         pd.ip_factor = d->ip_factor;
         pd.penalty_mode = d->penalty_mode;
         pd.local_solver = d->local_solver;
         pd.model = d->model;
-        mg->fp32_levels = mg->fp32_levels || pd.precision == TPSS_FP32;
         rc = tpss_precond_create(lv.L, lv.op, &pd, &lv.P);
         if(rc) fail(rc, tpss_last_error());
       }
@@ -710,7 +711,7 @@ void loop_body(tpss_mg *mg, cudaGraphConditionalHandle h, cudaStream_t s)
   vec_dot(n, r, top.x.ptr, mg->partial.ptr, d_rz_new, s);
   cg_update_p_loop<<<grid_for(n), 256, 0, s>>>(n, p, top.x.ptr, d_rz_new, d_rz, st);
   TPSS_CUDA(cudaMemcpyAsync(d_rz, d_rz_new, sizeof(double), cudaMemcpyDeviceToDevice, s));
-  operator_apply(top.op, Ap, p, s, nullptr, mg->fp32_levels);
+  operator_apply(top.op, Ap, p, s);
   vec_dot(n, p, Ap, mg->partial.ptr, d_pAp, s);
   cg_update_xr<<<grid_for(n), 256, 0, s>>>(n, u, r, p, Ap, d_rz, d_pAp);
   vec_dot(n, r, r, mg->partial.ptr, d_rr, s);
@@ -863,7 +864,7 @@ extern "C" int tpss_mg_cg_solve(tpss_mg *mg, double *u, const double *f, double 
       vec_dot(n, r, top.x.ptr, mg->partial.ptr, d_rz, s);
       for(it = 1; it <= max_iter; ++it)
       {
-        operator_apply(top.op, Ap, p, s, nullptr, mg->fp32_levels);
+        operator_apply(top.op, Ap, p, s);
         vec_dot(n, p, Ap, mg->partial.ptr, d_pAp, s);
         cg_update_xr<<<grid_for(n), 256, 0, s>>>(n, u, r, p, Ap, d_rz, d_pAp);
         vec_dot(n, r, r, mg->partial.ptr, d_rr, s);

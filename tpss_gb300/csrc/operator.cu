@@ -708,6 +708,11 @@ extern "C" int tpss_operator_create(const tpss_layout *layout, double ip_factor,
 extern "C" int tpss_operator_create_penalty(const tpss_layout *layout, double ip_factor, int penalty_mode,
                                             tpss_operator **out)
 {
+  return tpss::operator_create(layout, ip_factor, penalty_mode, true, out);
+}
+
+int tpss::operator_create(const tpss_layout *layout, double ip_factor, int penalty_mode, bool lines, tpss_operator **out)
+{
   return guarded([&] {
     TPSS_REQUIRE(layout && out, "null argument");
     TPSS_REQUIRE(ip_factor > 0.0, "ip_factor must be positive");
@@ -771,7 +776,7 @@ extern "C" int tpss_operator_create_penalty(const tpss_layout *layout, double ip
       op->d_fac32[d].upload(fac32.data(), fac32.size());
       op->nblk_cells[d] = layout->nc[d];
     }
-    build_op_lines(*op, *layout, pen);
+    if(lines) build_op_lines(*op, *layout, pen);
     *out = op.release();
   });
 }

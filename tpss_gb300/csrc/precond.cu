@@ -1109,7 +1109,9 @@ void smoother_steps(tpss_smoother *sm, double *x, const double *b, cudaStream_t 
   if(sm->tmp.n < (size_t)n) sm->tmp.resize(n);
   for(int k = 0; k < sm->n_steps; ++k)
   {
-    operator_apply(sm->op, sm->residual.ptr, x, s, b);  // r = b - A x
+    // (cell by cell next to an FP32 smoother, as in the multiplicative sweep: after 20 steps the line-by-line residual's
+    // rounding had moved x by up to 2.5e-9)
+    operator_apply(sm->op, sm->residual.ptr, x, s, b, sm->p->desc.precision == TPSS_FP32);  // r = b - A x
     precond_vmult(sm->p, sm->tmp.ptr, sm->residual.ptr, s);
     vec_axpby(n, sm->damping, sm->tmp.ptr, 1.0, x, s);  // x += damping P r
   }
