@@ -8,9 +8,10 @@
 // (M, L), the other nodes with their cell and its neighbours, or their cell. On a uniform grid all cells but
 // those next to the boundary have the same rows: a few classes of rows, held in shared memory, where the
 // lanes of a warp read one address.
-// Measured, 256^2 cells, K = 3 (767^2 values): x pass 48 -> 11.4 us, y pass 75 -> 15.3 us against a thread per
+// Measured, 256^2 cells, K = 3 (767^2 values): x pass 48 -> 12.6 us, y pass 75 -> 17.0 us against a thread per
 // node with FP64 bands (the x pass waited on its coefficients, 104 bytes apart from lane to lane, the y
-// pass on the FP64 pipe: 41 instructions of 64 clocks). With one unit for the whole window 11.1 and 14.0 us.
+// pass on the FP64 pipe: 41 instructions of 64 clocks). With one unit for the whole window and
+// without the low products 11.1 and 14.0 us.
 #pragma once
 
 #include <type_traits>
@@ -47,29 +48,21 @@ struct BandArgs
   double mixed;
 };
 
+// with the products of the low limbs: the bilaplacian's entries differ by a factor of 1e2 to 1e5, and its small
+// ones would lose them (k = 5, slowly varying vector: 1.03e-15 off without, 0.98e-15 with, as the FP64 bands)
 template<int LEN>
 __device__ __forceinline__ int64_t dot(const int2 *__restrict__ row, const int *xh, const int *xl)
 {
-  fx::Acc M, S;
-  const int4 *row4 = reinterpret_cast<const int4 *>(row);
+  int h[1][LEN], l[1][LEN];
 #pragma unroll
-  for(int j2 = 0; j2 < (LEN + 1) / 2; ++j2)
+  for(int i = 0; i < LEN; ++i)
   {
-    const int4 c = row4[j2];
-    if(j2 == 0) M.start(c.y, xl[0]);
-    else M.add(c.y, xl[2 * j2]);
-    M.add(c.x, xh[2 * j2]);
-    if(j2 == 0) S.start(c.y, xh[0]);
-    else S.add(c.y, xh[2 * j2]);
-    if(2 * j2 + 1 < LEN)
-    {
-      const int j = 2 * j2 + 1 < LEN ? 2 * j2 + 1 : 0;
-      M.add(c.w, xl[j]);
-      M.add(c.z, xh[j]);
-      S.add(c.w, xh[j]);
-    }
+    h[0][i] = xh[i];
+    l[0][i] = xl[i];
   }
-  return S.value() + (M.hi + (int)(M.lo >> 31));
+  int64_t y[1];
+  fx::row_dot<LEN, 1, true>(row, h, l, y);
+  return y[0];
 }
 
 // A window of W values in limbs: |x| < 2^58, so that up to 4 * 7 + 1 terms stay within the accumulators, with

@@ -7,12 +7,18 @@
 // cell) as 64-bit integers with one exponent per block (block floating point):
 //   value = x 2^e,  |x| < 2^59,  coefficient = c 2^-F,  sum_j |c_ij| <= 2^62 in every row i.
 // With signed 32-bit limbs x = xh 2^32 + xl, c = ch 2^32 + cl (xl, cl in [-2^31, 2^31)) a row's
-// sum is  sum_j c_ij x_j / 2^64 = sum ch xh + (sum ch xl + cl xh) / 2^32 + (cl xl, dropped):
-// three IMAD.WIDE per product, the dropped terms and the rounding stay below one unit 2^(e+64-F),
-// and the accumulators cannot overflow (|sum ch xh| < 2^60, |sum ch xl + cl xh| < 2^63 for up to
-// 16 terms).  After every contraction the block is shifted up again to 59 bits by the headroom
-// its largest value leaves, so one contraction's error is 2^-58 of (row sum of |c|) x (largest
-// |x| of the block), where an FP64 chain makes up to 2^-53 sum_j |c_ij x_j| per addition.
+// sum is  sum_j c_ij x_j / 2^64 = sum ch xh + (sum ch xl + cl xh) / 2^32 + sum cl xl / 2^64:
+// three IMAD.WIDE per product without the last sum, four with it, and the accumulators cannot overflow
+// (|sum ch xh| < 2^60, |sum ch xl + cl xh| < 2^63 for up to 16 terms).
+//
+// Error of a row of n terms, in units 2^(e+64-F): 1/2 from the rounding, and without the low products up to n/4
+// (each is a quarter unit at most; random rows of 5 to 16 terms are off by 1.2 to 1.4 at worst). The largest
+// |x| is 2^58 units and more, a row sum of |c| 2^61 to 2^62 (of the largest row), so that this is (n + 2) 2^-57 at most
+// of (largest row sum of |c|) x (largest |x| of the block). An FP64 chain makes up to n 2^-53 sum_j |c_ij x_j|. The two
+// differ in kind: this one is relative to the block's largest value and the matrix' largest row, and beats FP64's where all of a
+// block's values enter a row with coefficients of one magnitude. So a block holds no values that its rows do not contract,
+// and the C0IP bands, whose coefficients differ by up to 1e5, and the transfers keep the low products (LOW).
+// After every contraction the block is shifted up again to 59 bits by the headroom its largest value leaves.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -172,12 +178,12 @@ __device__ __forceinline__ int64_t mul_m61(int64_t x, int mh, int ml)
 
 // ---- coefficient rows: int2 (x: low limb, y: high limb), read as pairs
 // y[p] = sum_j c_j x_j / 2^64 of one row of H coefficients for P vectors x in limbs (the first H of L
-// values each)
-template<int H, int L, int P>
+// values each). LOW: with the products of the low limbs, less their last 4 bits, so that up to 31 terms fit
+template<int H, int L, int P, bool LOW = false>
 __device__ __forceinline__ void row_dot_n(const int2 *__restrict__ row, const int (&xh)[P][L], const int (&xl)[P][L],
                                           int64_t (&y)[P])
 {
-  Acc M[P], S[P];
+  Acc M[P], S[P], Q[P];
   const int4 *row4 = reinterpret_cast<const int4 *>(row);
 #pragma unroll
   for(int j2 = 0; j2 < (H + 1) / 2; ++j2)
@@ -186,6 +192,11 @@ __device__ __forceinline__ void row_dot_n(const int2 *__restrict__ row, const in
 #pragma unroll
     for(int p = 0; p < P; ++p)
     {
+      if constexpr(LOW)
+      {
+        if(j2 == 0) Q[p].start(c.x, xl[p][0] >> 4);
+        else Q[p].add(c.x, xl[p][2 * j2] >> 4);
+      }
       if(j2 == 0) M[p].start(c.y, xl[p][0]);
       else M[p].add(c.y, xl[p][2 * j2]);
       M[p].add(c.x, xh[p][2 * j2]);
@@ -198,6 +209,7 @@ __device__ __forceinline__ void row_dot_n(const int2 *__restrict__ row, const in
 #pragma unroll
       for(int p = 0; p < P; ++p)
       {
+        if constexpr(LOW) Q[p].add(c.z, xl[p][j] >> 4);
         M[p].add(c.w, xl[p][j]);
         M[p].add(c.z, xh[p][j]);
         S[p].add(c.w, xh[p][j]);
@@ -206,14 +218,18 @@ __device__ __forceinline__ void row_dot_n(const int2 *__restrict__ row, const in
   }
   // rounded to the nearest unit from M's low word (which also keeps its last product one instruction)
 #pragma unroll
-  for(int p = 0; p < P; ++p) y[p] = S[p].value() + (M[p].hi + (int)(M[p].lo >> 31));
+  for(int p = 0; p < P; ++p)
+  {
+    if constexpr(LOW) y[p] = S[p].value() + ((M[p].value() + (Q[p].value() >> 28) + (1ll << 31)) >> 32);
+    else y[p] = S[p].value() + (M[p].hi + (int)(M[p].lo >> 31));
+  }
 }
 
-template<int H, int P>
+template<int H, int P, bool LOW = false>
 __device__ __forceinline__ void row_dot(const int2 *__restrict__ row, const int (&xh)[P][H], const int (&xl)[P][H],
                                         int64_t (&y)[P])
 {
-  row_dot_n<H, H, P>(row, xh, xl, y);
+  row_dot_n<H, H, P, LOW>(row, xh, xl, y);
 }
 }  // namespace fx
 }  // namespace tpss
