@@ -473,8 +473,8 @@ void for_degree(int k, const F &f)
 }
 
 // Integer rows of the operator's bands (c0ip_band.cuh), one set per class of cells with equal rows. None
-// (n_cls = 0: the kernels by node run) when there are more classes than a launch holds or when an entry that
-// the integer kernels leave out is not zero.
+// (n_cls = 0: the kernels by node run) when there are more classes than a launch holds, when an entry that
+// the integer kernels leave out is not zero, or when the entries' magnitudes leave no room for the vectors'.
 template<int K>
 void build_band_tables(C0ipLevel &L, int nc, const std::vector<double> &M, const std::vector<double> &Lm,
                        const std::vector<double> &B)
@@ -497,6 +497,8 @@ void build_band_tables(C0ipLevel &L, int nc, const std::vector<double> &M, const
   L.FM = exponent(M);
   L.FL = exponent(Lm);
   L.FB = exponent(B);
+  for(int F : {L.FM, L.FL, L.FB})
+    if(std::abs(F - 62) > fx::kTableRange) return;
   std::map<std::vector<int64_t>, int> ids;
   std::vector<int32_t> cls(nc);
   std::vector<int64_t> tab;

@@ -88,7 +88,7 @@ struct Mag
   __device__ __forceinline__ int exponent() const
   {
     const int e = (int)(hi >> 20);
-    return e < 1023 - 300 || e > 1023 + 300 ? -1 : e;
+    return e < 1023 - fx::kRange || e > 1023 + fx::kRange ? -1 : e;
   }
 };
 

@@ -29,6 +29,10 @@ namespace tpss
 {
 namespace fx
 {
+// Exponents of a block's largest value that the kernels cover whose matrices have entries within 2^(+-kTableRange): a
+// result's unit 2^(e - 58 + 64 - F), |F - 62| <= kTableRange, stays a normal number
+constexpr int kRange = 800, kTableRange = 150;
+
 // 64-bit accumulator of 32 x 32-bit products. add() is one IMAD.WIDE: it is written with the carry
 // flag because ptxas splits the accumulation of mad.wide chains into products and separate 64-bit
 // additions (43 instead of 30 instructions per value of a 5 x 5 pair of contractions, 19.6 instead of

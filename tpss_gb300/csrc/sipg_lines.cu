@@ -79,8 +79,9 @@ int scale_of(const std::vector<long double> &t, int b, int rows, int len, int b2
   return 62 - e;
 }
 
+// false: the matrices' magnitudes leave no room for the vectors'
 template<int N>
-void build(tpss_operator &op, const tpss_layout &L, Penalty pen)
+bool build(tpss_operator &op, const tpss_layout &L, Penalty pen)
 {
   using T = OpTab<N>;
   static const ext::Element<N> s(make_shape_1d(N - 1));  // (0.1 ms and more in the 113 bits of an Arm host)
@@ -114,6 +115,8 @@ void build(tpss_operator &op, const tpss_layout &L, Penalty pen)
         const int F[3] = {scale_of(t, T::ME, T::HE, T::LME, T::MO, T::H, T::LMO),
                           scale_of(t, T::CE, T::HE, T::LCE, T::CO, T::H, T::LCO),
                           scale_of(t, T::TE, 1, T::LME, T::TO, 1, T::LMO)};
+        for(int f : F)
+          if(std::abs(f - 62) > fx::kTableRange) return false;
         for(int i = 0; i < T::SIZE; ++i)
         {
           const int f = i < T::CE ? F[0] : i < T::TE ? F[1] : F[2];
@@ -141,6 +144,7 @@ void build(tpss_operator &op, const tpss_layout &L, Penalty pen)
   if(buf.size() % 2) buf.push_back(0);  // table rows are read as 16-byte pairs
   O.off_tab = put(ti.data(), ti.size());
   O.tables.upload(buf.data(), buf.size());
+  return true;
 }
 
 template<int DIM, int N>
@@ -252,7 +256,9 @@ void build_op_lines(tpss_operator &op, const tpss_layout &L, Penalty pen)
   OpLines &O = op.lines;
   if(!O.buf.try_resize((size_t)L.n_dofs * (L.dim == 3 ? 4 : 2))) return;
   O.order.create();
-  for_size(L.np, [&](auto n) { build<decltype(n)::value>(op, L, pen); });
+  for_size(L.np, [&](auto n) {
+    if(!build<decltype(n)::value>(op, L, pen)) O.buf.release();
+  });
 }
 
 bool op_lines_apply(tpss_operator &op, double *dst, const double *src, cudaStream_t s, const double *rhs)

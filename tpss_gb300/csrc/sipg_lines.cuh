@@ -72,11 +72,10 @@ __device__ __forceinline__ double negated(double v)
   return __hiloint2double(__double2hiint(v) ^ (int)0x80000000u, __double2loint(v));
 }
 
-// exponent range of the integers (as for the smoother)
 __device__ __forceinline__ bool out_of_range(unsigned hm, unsigned lo)
 {
   const int e = (int)(hm >> 20);
-  return (e < 1023 - 300 || e > 1023 + 300) && (hm | lo) != 0;
+  return (e < 1023 - fx::kRange || e > 1023 + fx::kRange) && (hm | lo) != 0;
 }
 
 template<int CNT>

@@ -11,7 +11,7 @@
 // directions: its row of the matrix has a single entry, and the others do not see it. The
 // remaining rows have no zeros, so that what sets a pencil's unit enters all of its results: one pass's rounding
 // is 2^-58 of the pencil's largest value, and small values next to large ones keep their digits.
-// Values the integers do not cover (infinities, NaN, magnitudes outside 2^(+-300)) take FP64 passes, pencil by
+// Values the integers do not cover (infinities, NaN, magnitudes outside 2^(+-800)) take FP64 passes, pencil by
 // pencil.
 //
 // Measured, 16^3 coarse cells, k = 4 (4.1M fine values): prolongation 25 us, restriction 25.5 us, where the tree
@@ -115,7 +115,7 @@ __device__ __forceinline__ int64_t dot4(const int2 *__restrict__ row, const int 
 __device__ __forceinline__ int exponent(unsigned hi, unsigned lo)
 {
   const int e = (int)(hi >> 20);
-  return (hi | lo) == 0 ? 1023 : e < 1023 - 300 || e > 1023 + 300 ? -1 : e;
+  return (hi | lo) == 0 ? 1023 : e < 1023 - fx::kRange || e > 1023 + fx::kRange ? -1 : e;
 }
 __device__ __forceinline__ void magnitude(double v, unsigned &hi, unsigned &lo)
 {
