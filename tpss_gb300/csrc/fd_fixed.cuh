@@ -293,7 +293,6 @@ struct FixArgs
   const int2 *__restrict__ fix_eo;
   const int2 *__restrict__ fexp;      // per entry: F of S^T (x) and S (y), dense form
   const int2 *__restrict__ fexp_eo;
-  bool fp64_only;                     // every patch on the FP64 passes (indefinite local problems)
 };
 
 template<int DIM, int NCP, int K1>
@@ -436,7 +435,7 @@ __global__ void __maxnreg__((FixCfg<DIM, NCP, K1>::REGS))
     __syncthreads();
     int emax = (int)(ctl[CTL_EMAX] >> 20);
     const bool zero = ctl[CTL_EMAX] == 0 && ctl[CTL_LO] == 0;
-    const bool slow = fa.fp64_only || (!zero && (emax < 1023 - 300 || emax > 1023 + 300));
+    const bool slow = !zero && (emax < 1023 - 300 || emax > 1023 + 300);
     if(zero) emax = 1023;
     int ex = emax - 1023 - 58;  // exponent of the block's unit
     // --- S^T along x[, y] and the last direction

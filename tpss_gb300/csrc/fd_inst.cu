@@ -22,19 +22,21 @@ namespace tpss
 {
 namespace
 {
-// FP64: the contractions run on the integer pipe (fd_fixed.cuh)
+// FP64: the contractions run on the integer pipe (fd_fixed.cuh); where the tables rule that out (indefinite local
+// problems) the FP64 kernel does all patches: the integer one's own FP64 passes, which are there for single
+// patches out of range, take 1.1 to 1.4 times as long (cell patches, 2D k = 7, 20^2: 34.9 against 47.6 us)
 template<typename T, int DIM, int NCP, int K1>
 bool launch_one(const fd::KernelArgs &a, const FdLaunch &l, cudaStream_t s, int sms)
 {
   if constexpr(std::is_same_v<T, double>)
   {
+    if(l.fp64_only) return fd::launch<T, DIM, NCP, K1>(a, s, sms, l.variant);
     fd::FixArgs f;
     f.k = a;
     f.fix = l.fix;
     f.fix_eo = l.fix_eo;
     f.fexp = l.fexp;
     f.fexp_eo = l.fexp_eo;
-    f.fp64_only = l.fp64_only;
     return fd::launch_fixed<DIM, NCP, K1>(f, s, sms, l.variant);
   }
   else
