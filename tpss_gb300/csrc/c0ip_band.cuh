@@ -53,16 +53,14 @@ struct BandArgs
 template<int LEN>
 __device__ __forceinline__ int64_t dot(const int2 *__restrict__ row, const int *xh, const int *xl)
 {
-  int h[1][LEN], l[1][LEN];
+  int h[LEN], l[LEN];
 #pragma unroll
   for(int i = 0; i < LEN; ++i)
   {
-    h[0][i] = xh[i];
-    l[0][i] = xl[i];
+    h[i] = xh[i];
+    l[i] = xl[i];
   }
-  int64_t y[1];
-  fx::row_dot<LEN, 1, true>(row, h, l, y);
-  return y[0];
+  return fx::row_dot<LEN, true>(row, h, l);
 }
 
 // A window of W values in limbs: |x| < 2^58, so that up to 4 * 7 + 1 terms stay within the accumulators, with

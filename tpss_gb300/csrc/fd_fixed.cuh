@@ -45,11 +45,9 @@ struct FixCfg
   static constexpr int ES = B::ESIZE;  // 8-byte words per table slot
   static constexpr int PS = FixPad<DIM, N>::SIZE;
   static constexpr int CTL = 8;        // control words per patch
-  // pencils per thread
-  static constexpr int NPT = 1;
-  static constexpr int TPP = NPENCIL / NPT;  // threads per patch
+  static constexpr int TPP = NPENCIL;  // threads per patch: one per pencil
   static constexpr int MAX_THREADS = 512, MAX_SMEM = 200 * 1024, MAX_VARIANTS = 3;
-  // registers per thread: 24 warps per SM with two pencils of up to 16 values in limbs each
+  // registers per thread (24 to 32 warps per SM; a pencil of up to 16 values takes 2 per value in limbs)
   static constexpr int REGS = N >= 8 ? 80 : 64;
   static constexpr int SLOT_BYTES = PS * 8 + DIM * ES * 8 + NCELL * 12 + CTL * 4;
   static constexpr int PPC_MEM = (96 * 1024) / SLOT_BYTES > 0 ? (96 * 1024) / SLOT_BYTES : 1;
@@ -144,14 +142,13 @@ __device__ __forceinline__ void slot_reduce(unsigned *dst, unsigned v, bool acti
   }
 }
 
-// A thread's pencils along a direction, data[j][m STRIDE], m < N: their values (get(j, m), |.| < 2^59)
+// A pencil along a direction, data[m STRIDE], m < N: its values (get(m), |.| < 2^59)
 // are replaced by S^T x (FWD) or S x, |.| <= 2^58; ent: the slot's table, dense [S^T][S] or even/odd
 // [Se^T][So^T][Se][So]. Returns the OR of the results' magnitudes. The values are held as limbs in
 // registers and every result goes straight to shared memory, so that the rows can be a loop: an
 // unrolled kernel misses the instruction cache.
-template<int N, bool FWD, int STRIDE, int NPT, typename Get>
-__device__ __forceinline__ unsigned fix_pass(int64_t *const (&data)[NPT], const int2 *__restrict__ ent, bool sym,
-                                             const Get &get)
+template<int N, bool FWD, int STRIDE, typename Get>
+__device__ __forceinline__ unsigned fix_pass(int64_t *data, const int2 *__restrict__ ent, bool sym, const Get &get)
 {
   unsigned mag = 0;
   if constexpr(N % 2 == 0)
@@ -160,52 +157,39 @@ __device__ __forceinline__ unsigned fix_pass(int64_t *const (&data)[NPT], const 
     {
       using X = EoEntry<double, N>;
       constexpr int H = X::H, HP = X::HPAD;
-      int eh[NPT][H], el[NPT][H], oh[NPT][H], ol[NPT][H];
+      int eh[H], el[H], oh[H], ol[H];
 #pragma unroll
-      for(int j = 0; j < NPT; ++j)
-#pragma unroll
-        for(int i = 0; i < H; ++i)
-        {
-          // forward: sums and differences of mirrored values; backward: even and odd modes
-          const int64_t a = get(j, i), b = get(j, FWD ? N - 1 - i : H + i);
-          fx::split(FWD ? a + b : a, eh[j][i], el[j][i]);
-          fx::split(FWD ? a - b : b, oh[j][i], ol[j][i]);
-        }
+      for(int i = 0; i < H; ++i)
+      {
+        // forward: sums and differences of mirrored values; backward: even and odd modes
+        const int64_t a = get(i), b = get(FWD ? N - 1 - i : H + i);
+        fx::split(FWD ? a + b : a, eh[i], el[i]);
+        fx::split(FWD ? a - b : b, oh[i], ol[i]);
+      }
       const int2 *re = ent + (FWD ? 0 : X::SE), *ro = ent + (FWD ? X::SOT : X::SO);
 #pragma unroll kFixUnroll
       for(int k = 0; k < H; ++k)
       {
-        int64_t e[NPT], o[NPT];
-        fx::row_dot<H, NPT>(re + k * HP, eh, el, e);
-        fx::row_dot<H, NPT>(ro + k * HP, oh, ol, o);
-#pragma unroll
-        for(int j = 0; j < NPT; ++j)
-        {
-          const int64_t y0 = FWD ? e[j] : e[j] + o[j], y1 = FWD ? o[j] : e[j] - o[j];
-          data[j][k * STRIDE] = y0;
-          data[j][(FWD ? H + k : N - 1 - k) * STRIDE] = y1;
-          mag |= fx::mag_hi(y0) | fx::mag_hi(y1);
-        }
+        const int64_t e = fx::row_dot<H>(re + k * HP, eh, el), o = fx::row_dot<H>(ro + k * HP, oh, ol);
+        const int64_t y0 = FWD ? e : e + o, y1 = FWD ? o : e - o;
+        data[k * STRIDE] = y0;
+        data[(FWD ? H + k : N - 1 - k) * STRIDE] = y1;
+        mag |= fx::mag_hi(y0) | fx::mag_hi(y1);
       }
       return mag;
     }
   }
   constexpr int NP = Entry<double, N>::NPAD;
   const int2 *row = ent + (FWD ? Entry<double, N>::ST : Entry<double, N>::S);
+  int h[N], l[N];
 #pragma unroll
-  for(int j = 0; j < NPT; ++j)
-  {
-    int h[1][N], l[1][N];
-#pragma unroll
-    for(int i = 0; i < N; ++i) fx::split(get(j, i), h[0][i], l[0][i]);
+  for(int i = 0; i < N; ++i) fx::split(get(i), h[i], l[i]);
 #pragma unroll kFixUnroll
-    for(int i = 0; i < N; ++i)
-    {
-      int64_t y[1];
-      fx::row_dot<N, 1>(row + i * NP, h, l, y);
-      data[j][i * STRIDE] = y[0];
-      mag |= fx::mag_hi(y[0]);
-    }
+  for(int i = 0; i < N; ++i)
+  {
+    const int64_t y = fx::row_dot<N>(row + i * NP, h, l);
+    data[i * STRIDE] = y;
+    mag |= fx::mag_hi(y);
   }
   return mag;
 }
@@ -302,7 +286,7 @@ __global__ void __maxnreg__((FixCfg<DIM, NCP, K1>::REGS))
   using C = FixCfg<DIM, NCP, K1>;
   using P = FixPad<DIM, C::N>;
   constexpr int N = C::N, NLOC = C::NLOC, NCELL = C::NCELL, CELLDOFS = C::CELLDOFS, ES = C::ES, NPENCIL = C::NPENCIL;
-  constexpr int NPT = C::NPT, TPP = C::TPP;
+  constexpr int TPP = C::TPP;
   constexpr int SX = P::SX, SXY = P::SXY, PS = C::PS;
   const KernelArgs &a = fa.k;
   const int PPC = a.ppc, NTHR = blockDim.x;
@@ -339,16 +323,11 @@ __global__ void __maxnreg__((FixCfg<DIM, NCP, K1>::REGS))
     }
     s_map[i] = (unsigned)off | (unsigned)cn << 13 | (unsigned)e << 16;
   }
-  // pencils q + j TPP of this thread: x along (y, z), y along (x, z), last direction
-  int bx[NPT], by[NPT], bz[NPT];
-#pragma unroll
-  for(int j = 0; j < NPT; ++j)
-  {
-    const int p = q + j * TPP, pa = p % N, pb = p / N;
-    bx[j] = DIM == 2 ? SX * p : SX * pa + SXY * pb;
-    by[j] = DIM == 2 ? p : pa + SXY * pb;
-    bz[j] = pa + SX * pb;  // 3D
-  }
+  // this thread's pencils: x along (y, z), y along (x, z), last direction
+  const int pa = q % N, pb = q / N;
+  const int bx = DIM == 2 ? SX * q : SX * pa + SXY * pb;
+  const int by = DIM == 2 ? q : pa + SXY * pb;
+  const int bz = pa + SX * pb;  // 3D
   for(int i = tid; i < PPC * DIM; i += NTHR) s_code[i] = -1;
   __syncthreads();
 
@@ -398,23 +377,19 @@ __global__ void __maxnreg__((FixCfg<DIM, NCP, K1>::REGS))
       unsigned hm = 0, lo = 0;
       if(active)
       {
+        double v[N];
 #pragma unroll
-        for(int j0 = 0; j0 < N * NPT; j0 += N)
+        for(int j = 0; j < N; ++j)
         {
-          double v[N];
+          const unsigned m = s_map[q + j * TPP];
+          v[j] = a.src[s_first[sl * NCELL + ((m >> 13) & 7)] + (m >> 16)];
+        }
 #pragma unroll
-          for(int j = 0; j < N; ++j)
-          {
-            const unsigned m = s_map[q + (j0 + j) * TPP];
-            v[j] = a.src[s_first[sl * NCELL + ((m >> 13) & 7)] + (m >> 16)];
-          }
-#pragma unroll
-          for(int j = 0; j < N; ++j)
-          {
-            my[s_map[q + (j0 + j) * TPP] & 0x1fff] = __double_as_longlong(v[j]);
-            hm = max(hm, (unsigned)__double2hiint(v[j]) & 0x7fffffffu);
-            lo |= (unsigned)__double2loint(v[j]);
-          }
+        for(int j = 0; j < N; ++j)
+        {
+          my[s_map[q + j * TPP] & 0x1fff] = __double_as_longlong(v[j]);
+          hm = max(hm, (unsigned)__double2hiint(v[j]) & 0x7fffffffu);
+          lo |= (unsigned)__double2loint(v[j]);
         }
       }
       slot_reduce<TPP, true>(ctl + CTL_EMAX, hm, active, uniform);
@@ -441,9 +416,7 @@ __global__ void __maxnreg__((FixCfg<DIM, NCP, K1>::REGS))
     // --- S^T along x[, y] and the last direction
     auto forward = [&](auto dir) {
       constexpr int d = decltype(dir)::value, STRIDE = d == 0 ? 1 : d == 1 ? SX : SXY;
-      int64_t *p[NPT];
-#pragma unroll
-      for(int j = 0; j < NPT; ++j) p[j] = my + (d == 0 ? bx[j] : d == 1 ? by[j] : bz[j]);
+      int64_t *p = my + (d == 0 ? bx : d == 1 ? by : bz);
       const int s = d == 0 ? 0 : fx::headroom(ctl[CTL_OR0 + (d > 0 ? d - 1 : 0)]);
       const bool sy = code[d] & 1;
       unsigned mag = 0;
@@ -452,14 +425,13 @@ __global__ void __maxnreg__((FixCfg<DIM, NCP, K1>::REGS))
         if(slow)
         {
           const int e = code[d] >> 1;
-          for(int j = 0; j < NPT; ++j)
-            slow_pass<N, true>(myd + (d == 0 ? bx[j] : d == 1 ? by[j] : bz[j]), STRIDE,
-                               sy ? fd_eo + (size_t)e * a.eo_stride : fd + (size_t)e * a.entry_stride, sy, 1.0);
+          slow_pass<N, true>(reinterpret_cast<double *>(p), STRIDE,
+                             sy ? fd_eo + (size_t)e * a.eo_stride : fd + (size_t)e * a.entry_stride, sy, 1.0);
         }
         else
-          mag = fix_pass<N, true, STRIDE, NPT>(p, ent + d * ES, sy, [&](int j, int m) {
-            if constexpr(d == 0) return fx::from_double(__longlong_as_double(p[j][m]), emax);
-            else return fx::shl(p[j][m * STRIDE], s);
+          mag = fix_pass<N, true, STRIDE>(p, ent + d * ES, sy, [&](int m) {
+            if constexpr(d == 0) return fx::from_double(__longlong_as_double(p[m]), emax);
+            else return fx::shl(p[m * STRIDE], s);
           });
       }
       ex += 64 - ex2[d].x - s;
@@ -474,51 +446,47 @@ __global__ void __maxnreg__((FixCfg<DIM, NCP, K1>::REGS))
     if constexpr(DIM == 3) forward(std::integral_constant<int, 2>{});
     // --- times the reciprocal eigenvalue sums (the thread's own pencil of the last direction)
     constexpr int L = DIM - 1, LSTR = DIM == 2 ? SX : SXY;
-    int g[NPT];  // exponents of the pencils' products
+    int g = 0;  // exponent of the pencil's products
     unsigned xb = 0;
     if(active)
     {
       const double *lamL = reinterpret_cast<const double *>(ent + L * ES) +
                            ((code[L] & 1) ? EoEntry<double, N>::LAM : Entry<double, N>::LAM);
-#pragma unroll
-      for(int j = 0; j < NPT; ++j)
+      int64_t *v = my + (DIM == 2 ? by : bz);
+      const double *rt = rcp_tab ? rcp_tab + (size_t)s_combo[sl] * NLOC + q : nullptr;
+      double lsum = 0.0;
+      if(!rt)
       {
-        const int p = q + j * TPP;
-        int64_t *v = my + (DIM == 2 ? by[j] : bz[j]);
-        const double *rt = rcp_tab ? rcp_tab + (size_t)s_combo[sl] * NLOC + p : nullptr;
-        double lsum = 0.0;
-        if(!rt)
-        {
-          int rem = p;
+        int rem = q;
 #pragma unroll
-          for(int d = 0; d < DIM - 1; ++d)
-          {
-            const int lam = (code[d] & 1) ? EoEntry<double, N>::LAM : Entry<double, N>::LAM;
-            lsum += reinterpret_cast<const double *>(ent)[d * ES + lam + rem % N];
-            rem /= N;
-          }
-        }
-        if(slow)
+        for(int d = 0; d < DIM - 1; ++d)
         {
-          double *o = reinterpret_cast<double *>(v);
-#pragma unroll 1
-          for(int i = 0; i < N; ++i)
-          {
-            if(rt) o[i * LSTR] *= __ldg(rt + i * NPENCIL);
-            else o[i * LSTR] = o[i * LSTR] / (lsum + lamL[i]);
-          }
-          continue;
+          const int lam = (code[d] & 1) ? EoEntry<double, N>::LAM : Entry<double, N>::LAM;
+          lsum += reinterpret_cast<const double *>(ent)[d * ES + lam + rem % N];
+          rem /= N;
         }
+      }
+      if(slow)
+      {
+        double *o = reinterpret_cast<double *>(v);
+#pragma unroll 1
+        for(int i = 0; i < N; ++i)
+        {
+          if(rt) o[i * LSTR] *= __ldg(rt + i * NPENCIL);
+          else o[i * LSTR] = o[i * LSTR] / (lsum + lamL[i]);
+        }
+      }
+      else
+      {
         bool any;
-        const int e59 = scale_by_reciprocals<N, LSTR>(
+        g = scale_by_reciprocals<N, LSTR>(
           v,
-          [&](int i, int &mh, int &ml, int &q) {
-            if(rt) fx::split_positive(__ldg(rt + i * NPENCIL), mh, ml, q);
-            else fx::reciprocal(lsum + lamL[i], mh, ml, q);
+          [&](int i, int &mh, int &ml, int &e) {
+            if(rt) fx::split_positive(__ldg(rt + i * NPENCIL), mh, ml, e);
+            else fx::reciprocal(lsum + lamL[i], mh, ml, e);
           },
           any);
-        g[j] = e59;
-        if(any) xb = max(xb, (unsigned)(e59 + 59 + kExpBias));
+        if(any) xb = (unsigned)(g + 59 + kExpBias);
       }
     }
     slot_reduce<TPP, true>(ctl + CTL_X, xb, active, uniform);
@@ -529,9 +497,7 @@ __global__ void __maxnreg__((FixCfg<DIM, NCP, K1>::REGS))
     ex += 61 + G;
     auto backward = [&](auto dir) {
       constexpr int d = decltype(dir)::value, STRIDE = d == 0 ? 1 : d == 1 ? SX : SXY;
-      int64_t *p[NPT];
-#pragma unroll
-      for(int j = 0; j < NPT; ++j) p[j] = my + (d == 0 ? bx[j] : d == 1 ? by[j] : bz[j]);
+      int64_t *p = my + (d == 0 ? bx : d == 1 ? by : bz);
       const int s = d == L ? 0 : fx::headroom(ctl[CTL_OR0 + DIM - 2 + L - d]);
       const bool sy = code[d] & 1;
       unsigned mag = 0;
@@ -540,15 +506,14 @@ __global__ void __maxnreg__((FixCfg<DIM, NCP, K1>::REGS))
         if(slow)
         {
           const int e = code[d] >> 1;
-          for(int j = 0; j < NPT; ++j)
-            slow_pass<N, false>(myd + (d == 0 ? bx[j] : d == 1 ? by[j] : bz[j]), STRIDE,
-                                sy ? fd_eo + (size_t)e * a.eo_stride : fd + (size_t)e * a.entry_stride, sy,
-                                d == 0 ? a.omega : 1.0);
+          slow_pass<N, false>(reinterpret_cast<double *>(p), STRIDE,
+                              sy ? fd_eo + (size_t)e * a.eo_stride : fd + (size_t)e * a.entry_stride, sy,
+                              d == 0 ? a.omega : 1.0);
         }
         else
           // the last direction's pencils come down to the block's exponent
-          mag = fix_pass<N, false, STRIDE, NPT>(p, ent + d * ES, sy, [&](int j, int m) {
-            return d == L ? fx::shr_s(p[j][m * STRIDE], G - g[j]) : fx::shl(p[j][m * STRIDE], s);
+          mag = fix_pass<N, false, STRIDE>(p, ent + d * ES, sy, [&](int m) {
+            return d == L ? fx::shr_s(p[m * STRIDE], G - g) : fx::shl(p[m * STRIDE], s);
           });
       }
       ex += 64 - ex2[d].y - s;
@@ -567,7 +532,7 @@ __global__ void __maxnreg__((FixCfg<DIM, NCP, K1>::REGS))
       const double sc = slow ? 1.0 : far ? a.omega : a.omega * fx::pow2(ex);
       constexpr int CH = N % 5 == 0 ? 5 : N % 4 == 0 ? 4 : N % 7 == 0 ? 7 : N % 3 == 0 ? 3 : N;
 #pragma unroll 1
-      for(int j0 = 0; j0 < N * NPT; j0 += CH)
+      for(int j0 = 0; j0 < N; j0 += CH)
       {
         double old[CH];
         double *at[CH];

@@ -145,7 +145,7 @@ __device__ __forceinline__ void split_positive(double r, int &mh, int &ml, int &
 
 // 1/d = m 2^q with 2^60 <= m <= 2^61, in the form of split_positive: Newton's iteration r <- r + r (1 - d r) from a
 // single-precision start, twice (24 to 48 to 61 bits). An FP64 division keeps a warp's FP64 pipe busy for
-// some 10 instructions of 64 clocks (Richardson step on 20^3 distorted cells, k = 3: 432 -> 425 us). What is not in (2^-900, 2^900) is divided in FP64.
+// some 10 instructions of 64 clocks (Richardson step on 20^3 distorted cells, k = 3: 432 -> 424 us). What is not in (2^-900, 2^900) is divided in FP64.
 __device__ __forceinline__ void reciprocal(double d, int &mh, int &ml, int &q)
 {
   const int hi = __double2hiint(d), e = hi >> 20;
@@ -181,59 +181,39 @@ __device__ __forceinline__ int64_t mul_m61(int64_t x, int mh, int ml)
 }
 
 // ---- coefficient rows: int2 (x: low limb, y: high limb), read as pairs
-// y[p] = sum_j c_j x_j / 2^64 of one row of H coefficients for P vectors x in limbs (the first H of L
-// values each). LOW: with the products of the low limbs, less their last 4 bits, so that up to 31 terms fit
-template<int H, int L, int P, bool LOW = false>
-__device__ __forceinline__ void row_dot_n(const int2 *__restrict__ row, const int (&xh)[P][L], const int (&xl)[P][L],
-                                          int64_t (&y)[P])
+// sum_j c_j x_j / 2^64 of one row of H coefficients for the first H of L values x in limbs. LOW: with the
+// products of the low limbs, less their last 4 bits, so that up to 31 terms fit
+template<int H, bool LOW = false, int L>
+__device__ __forceinline__ int64_t row_dot(const int2 *__restrict__ row, const int (&xh)[L], const int (&xl)[L])
 {
-  Acc M[P], S[P], Q[P];
+  Acc M, S, Q;
   const int4 *row4 = reinterpret_cast<const int4 *>(row);
 #pragma unroll
   for(int j2 = 0; j2 < (H + 1) / 2; ++j2)
   {
     const int4 c = row4[j2];
-#pragma unroll
-    for(int p = 0; p < P; ++p)
+    if constexpr(LOW)
     {
-      if constexpr(LOW)
-      {
-        if(j2 == 0) Q[p].start(c.x, xl[p][0] >> 4);
-        else Q[p].add(c.x, xl[p][2 * j2] >> 4);
-      }
-      if(j2 == 0) M[p].start(c.y, xl[p][0]);
-      else M[p].add(c.y, xl[p][2 * j2]);
-      M[p].add(c.x, xh[p][2 * j2]);
-      if(j2 == 0) S[p].start(c.y, xh[p][0]);
-      else S[p].add(c.y, xh[p][2 * j2]);
+      if(j2 == 0) Q.start(c.x, xl[0] >> 4);
+      else Q.add(c.x, xl[2 * j2] >> 4);
     }
+    if(j2 == 0) M.start(c.y, xl[0]);
+    else M.add(c.y, xl[2 * j2]);
+    M.add(c.x, xh[2 * j2]);
+    if(j2 == 0) S.start(c.y, xh[0]);
+    else S.add(c.y, xh[2 * j2]);
     if(2 * j2 + 1 < H)
     {
       const int j = 2 * j2 + 1 < H ? 2 * j2 + 1 : 0;
-#pragma unroll
-      for(int p = 0; p < P; ++p)
-      {
-        if constexpr(LOW) Q[p].add(c.z, xl[p][j] >> 4);
-        M[p].add(c.w, xl[p][j]);
-        M[p].add(c.z, xh[p][j]);
-        S[p].add(c.w, xh[p][j]);
-      }
+      if constexpr(LOW) Q.add(c.z, xl[j] >> 4);
+      M.add(c.w, xl[j]);
+      M.add(c.z, xh[j]);
+      S.add(c.w, xh[j]);
     }
   }
   // rounded to the nearest unit from M's low word (which also keeps its last product one instruction)
-#pragma unroll
-  for(int p = 0; p < P; ++p)
-  {
-    if constexpr(LOW) y[p] = S[p].value() + ((M[p].value() + (Q[p].value() >> 28) + (1ll << 31)) >> 32);
-    else y[p] = S[p].value() + (M[p].hi + (int)(M[p].lo >> 31));
-  }
-}
-
-template<int H, int P, bool LOW = false>
-__device__ __forceinline__ void row_dot(const int2 *__restrict__ row, const int (&xh)[P][H], const int (&xl)[P][H],
-                                        int64_t (&y)[P])
-{
-  row_dot_n<H, H, P, LOW>(row, xh, xl, y);
+  if constexpr(LOW) return S.value() + ((M.value() + (Q.value() >> 28) + (1ll << 31)) >> 32);
+  else return S.value() + (M.hi + (int)(M.lo >> 31));
 }
 }  // namespace fx
 }  // namespace tpss

@@ -2,8 +2,8 @@
 //
 // Layers: n_in -> n_hidden (tanh) -> ... -> n_hidden (tanh) -> n_out (linear), FP32. The
 // widths are small (tens of units), so every layer is a tiled CUDA-core product with a fixed
-// summation order; the products are far too small for tensor-core tiles to pay, and FP32 results
-// would need several of them.
+// summation order. A mini-batch's products are far too small for tensor-core tiles; those of a whole level's patches
+// (tens of thousands of rows) are not, but FP32 results would take several tensor-core products each.
 // Training minimizes the mean squared error over all outputs with Adam (Kingma & Ba 2015:
 // beta1 0.9, beta2 0.999, eps 1e-8, bias-corrected moments), mini-batches in a seeded
 // permutation per epoch.
@@ -45,7 +45,7 @@ constexpr int kLossBlocks = 256;
 // grid layer each, whose partial results wgrad_reduce_kernel adds in ascending order: both orders are
 // fixed. For the local-solver network (29,791 rows, 87-64-64-64-108) one forward pass and one gradient
 // took 12.7 ms with a thread per result (the weight gradient's threads walked all rows, the others
-// read the weights uncoalesced); now 0.42 ms, 19 to 25 us per product (about 20 TFLOP/s, bound by
+// read the weights uncoalesced); now 0.47 ms, 19 to 25 us per product (about 20 TFLOP/s, bound by
 // shared-memory reads). Large tiles below num_sms() * 64 rows would leave SMs empty.
 enum GemmOp
 {

@@ -91,18 +91,18 @@ __device__ __forceinline__ void magnitude(const double (&v)[CNT], unsigned &hm, 
 
 // even and odd parts of a pencil in limbs: eh/el[0 .. HE) (pair sums, then the middle node), oh/ol
 template<int N, int LE, int LO>
-__device__ __forceinline__ void split_parts(const double (&u)[N], int emax, int (&eh)[1][LE], int (&el)[1][LE],
-                                            int (&oh)[1][LO], int (&ol)[1][LO])
+__device__ __forceinline__ void split_parts(const double (&u)[N], int emax, int (&eh)[LE], int (&el)[LE], int (&oh)[LO],
+                                            int (&ol)[LO])
 {
   constexpr int H = N / 2;
 #pragma unroll
   for(int j = 0; j < H; ++j)
   {
     const int64_t a = fx::from_double(u[j], emax), b = fx::from_double(u[N - 1 - j], emax);
-    fx::split(a + b, eh[0][j], el[0][j]);
-    fx::split(a - b, oh[0][j], ol[0][j]);
+    fx::split(a + b, eh[j], el[j]);
+    fx::split(a - b, oh[j], ol[j]);
   }
-  if constexpr(N % 2 == 1) fx::split(fx::from_double(u[H], emax), eh[0][H], el[0][H]);
+  if constexpr(N % 2 == 1) fx::split(fx::from_double(u[H], emax), eh[H], el[H]);
 }
 
 // One pencil of a cell. In: q (and p) of the cell, the neighbours' face values uL, uR. Out: r without
@@ -190,15 +190,13 @@ __device__ __forceinline__ void cell_pencil(const int2 *__restrict__ tab, const 
   // (a zero pencil takes the unit of its neighbours)
   const int en = (int)(hn >> 20), eq = hq != 0 ? (int)(hq >> 20) : hn != 0 ? en : 1023, ep = hp == 0 ? 1023 : (int)(hp >> 20);
   // limbs of the even parts and s, and of the odd parts and d
-  int eh[1][HE + 1], el[1][HE + 1], oh[1][H + 1], ol[1][H + 1];
+  int eh[HE + 1], el[HE + 1], oh[H + 1], ol[H + 1];
   split_parts<N>(q, eq, eh, el, oh, ol);
   const int uq = eq - 1023 - 58 + 64;
   {
-    int64_t te[1], to[1];
-    fx::row_dot_n<HE, HE + 1, 1>(tab + T::TE, eh, el, te);
-    fx::row_dot_n<H, H + 1, 1>(tab + T::TO, oh, ol, to);
-    tu = fx::to_double_alu(te[0] + to[0], uq - FT);
-    tl = fx::to_double_alu(te[0] - to[0], uq - FT);
+    const int64_t te = fx::row_dot<HE>(tab + T::TE, eh, el), to = fx::row_dot<H>(tab + T::TO, oh, ol);
+    tu = fx::to_double_alu(te + to, uq - FT);
+    tl = fx::to_double_alu(te - to, uq - FT);
   }
   if constexpr(PARTS)
   {
@@ -206,37 +204,27 @@ __device__ __forceinline__ void cell_pencil(const int2 *__restrict__ tab, const 
     const bool far = en > eq + 2;
     {
       const int64_t lo = far ? 0 : fx::from_double(uL, eq + 2) << 2, hi = far ? 0 : fx::from_double(uR, eq + 2) << 2;
-      fx::split(hi + lo, eh[0][HE], el[0][HE]);
-      fx::split(hi - lo, oh[0][H], ol[0][H]);
+      fx::split(hi + lo, eh[HE], el[HE]);
+      fx::split(hi - lo, oh[H], ol[H]);
     }
-    int ph[1][HE + 1], pl[1][HE + 1], sh[1][H + 1], sl[1][H + 1];
+    int ph[HE + 1], pl[HE + 1], sh[H + 1], sl[H + 1];
     if constexpr(HAS_P) split_parts<N>(p, ep, ph, pl, sh, sl);
     // the two contributions to r come to the coarser of their units (a zero one has none)
     const int u2 = ep - 1023 - 58 + 64 - FM, u1 = HAS_P && (hq | hn) == 0 ? u2 : uq - FC;
     const int U = HAS_P && hp != 0 ? max(u1, u2) : u1;
     auto even = [&](int i) {
-      int64_t a[1];
-      fx::row_dot_n<HE + 1, HE + 1, 1>(tab + T::CE + i * T::LCE, eh, el, a);
+      const int64_t a = fx::row_dot<HE + 1>(tab + T::CE + i * T::LCE, eh, el);
       if constexpr(HAS_P)
-      {
-        int64_t b[1];
-        fx::row_dot_n<HE, HE + 1, 1>(tab + T::ME + i * T::LME, ph, pl, b);
-        return fx::shr_s(a[0], U - u1) + fx::shr_s(b[0], max(U - u2, 0));
-      }
+        return fx::shr_s(a, U - u1) + fx::shr_s(fx::row_dot<HE>(tab + T::ME + i * T::LME, ph, pl), max(U - u2, 0));
       else
-        return a[0];
+        return a;
     };
     auto odd = [&](int i) {
-      int64_t a[1];
-      fx::row_dot_n<H + 1, H + 1, 1>(tab + T::CO + i * T::LCO, oh, ol, a);
+      const int64_t a = fx::row_dot<H + 1>(tab + T::CO + i * T::LCO, oh, ol);
       if constexpr(HAS_P)
-      {
-        int64_t b[1];
-        fx::row_dot_n<H, H + 1, 1>(tab + T::MO + i * T::LMO, sh, sl, b);
-        return fx::shr_s(a[0], U - u1) + fx::shr_s(b[0], max(U - u2, 0));
-      }
+        return fx::shr_s(a, U - u1) + fx::shr_s(fx::row_dot<H>(tab + T::MO + i * T::LMO, sh, sl), max(U - u2, 0));
       else
-        return a[0];
+        return a;
     };
 #pragma unroll
     for(int i = 0; i < H; ++i)
@@ -263,11 +251,10 @@ __device__ __forceinline__ void cell_pencil(const int2 *__restrict__ tab, const 
 #pragma unroll
       for(int i = 0; i < HE; ++i)
       {
-        int64_t e[1], o[1] = {0};
-        fx::row_dot_n<HE, HE + 1, 1>(tab + T::ME + i * T::LME, eh, el, e);
-        if(i < H) fx::row_dot_n<H, H + 1, 1>(tab + T::MO + i * T::LMO, oh, ol, o);
-        m[i] = fx::to_double_alu(e[0] + o[0], uq - FM);
-        if(i < H) m[N - 1 - i] = fx::to_double_alu(e[0] - o[0], uq - FM);
+        const int64_t e = fx::row_dot<HE>(tab + T::ME + i * T::LME, eh, el);
+        const int64_t o = i < H ? fx::row_dot<H>(tab + T::MO + i * T::LMO, oh, ol) : 0;
+        m[i] = fx::to_double_alu(e + o, uq - FM);
+        if(i < H) m[N - 1 - i] = fx::to_double_alu(e - o, uq - FM);
       }
     }
   }

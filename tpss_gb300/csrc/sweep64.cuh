@@ -101,8 +101,7 @@ __device__ __forceinline__ void transform(const double (&v)[N], int64_t *col, co
     fd::slow_pass<N, FWD>(out, STRIDE, sy ? t.fd_eo + (size_t)e * t.es_eo : t.fd + (size_t)e * t.es, sy, 1.0);
     return;
   }
-  int64_t *const c[1] = {col};
-  fd::fix_pass<N, FWD, STRIDE, 1>(c, slot, sy, [&](int, int m) { return fx::from_double(v[m], emax); });
+  fd::fix_pass<N, FWD, STRIDE>(col, slot, sy, [&](int m) { return fx::from_double(v[m], emax); });
   const int ex = emax - 1023 - 58 + 64 - F;
 #pragma unroll
   for(int m = 0; m < N; ++m) out[m * STRIDE] = fx::to_double(col[m * STRIDE], ex);
@@ -226,14 +225,13 @@ __global__ void __launch_bounds__(kLineThreads, K1 <= 5 ? 6 : 4) line_kernel(Lin
         }
         else
         {
-          int64_t *const cp[1] = {col};
-          fd::fix_pass<N, true, BT, 1>(cp, s_tab, sy, [&](int, int m) { return fx::from_double(x[m], emax); });
+          fd::fix_pass<N, true, BT>(col, s_tab, sy, [&](int m) { return fx::from_double(x[m], emax); });
           int ex = emax - 1023 - 58 + 64 - F.x;
           ex += 61 + fd::scale_by_reciprocals<N, BT>(col, [&](int i, int &mh, int &ml, int &q) {
             // (levels without the table are rare; fx::reciprocal here cost the others 1.7 %)
             fx::split_positive(r_tab ? __ldg(r_tab + i * RS) : 1.0 / (lxy + lam[i]), mh, ml, q);
           });
-          fd::fix_pass<N, false, BT, 1>(cp, s_tab, sy, [&](int, int m) { return col[m * BT]; });
+          fd::fix_pass<N, false, BT>(col, s_tab, sy, [&](int m) { return col[m * BT]; });
           ex += 64 - F.y;
 #pragma unroll
           for(int m = 0; m < N; ++m) cold[m * BT] = fx::to_double(col[m * BT], ex);
