@@ -31,7 +31,7 @@ def layout(tpss, dim, k, nc, patch=1):
     return tpss.SubdomainHandler(tpss.SubdomainHandler.AdditionalData(dim=dim, degree=k, n_cells=nc, patch_variant=patch))
 
 
-@pytest.mark.parametrize("dim,k,nc", [(2, 3, (24, 25)), (2, 5, (9, 11)), (2, 6, (9, 8)), (2, 7, (8, 7)), (3, 3, (9, 11, 9)),
+@pytest.mark.parametrize("dim,k,nc", [(2, 3, (24, 25)), (2, 5, (9, 11)), (2, 6, (9, 8)), (2, 7, (8, 7)), (3, 3, (11, 11, 10)),
                                       (3, 4, (3, 10, 9)), (3, 5, (5, 4, 5)), (3, 7, (4, 3, 4))])
 def test_operator(tpss, cuda, dim, k, nc):
     import torch

@@ -235,14 +235,15 @@ void for_size(int np, const F &f)
 }
 }  // namespace
 
-// Whether the passes are faster than the cell-wise kernel. On small levels both are latency: the passes take 12.4
-// (2D) and 18.6 us (3D) whatever the degree, the cell-wise kernel 9, 11.5 and 14.5 us for k = 1, 2, 3 in 2D and
-// 10.4, 13.8, 14.8, 18 and 21 us for k = 1 .. 5 in 3D; beyond that its multiply-adds cost 1.7 us per million
-// (2 per clock and SM), the passes' about 0.28 of that. The lines below are where the two meet
-// (measured equal: 2D k = 1 160^2 cells, 14.4 and 14.5 us; 3D k = 4 6^3, 18.6 and 19.1)
+// Whether the passes are faster than the cell-wise kernel. On small levels both are latency: replayed in a graph the
+// passes take 8 to 11 us in 2D and 13 to 20 us in 3D, the cell-wise kernel 6 to 10, 8 to 12 and 10 to 15 us for k = 1, 2, 3 in 2D
+// and 9, 12, 14, 17 and 20 us for k = 1 .. 5 in 3D; beyond that its multiply-adds cost 1.7 us per million
+// (2 per clock and SM), the passes' about 0.28 of that. The lines below are where the two meet. Measured, cell-wise and
+// passes: 2D k = 1 160^2 cells 12.1 and 12.4 us; 3D k = 1 24^3 15.2 and 17.3, 28^3 23.1 and 20.6; k = 2 16^3 16.2 and 16.4, 20^3
+// 25.2 and 20.5; k = 3 10^3 14.8 and 15.6, 12^3 19.2 and 16.2; k = 4 5^3 17.0 and 16.5
 static bool lines_pay(const tpss_layout &L)
 {
-  static const double from[2][8] = {{0, 4.6, 1.4, 0, 0, 0, 0, 0}, {0, 11.3, 7.8, 4.3, 0.8, 0, 0, 0}};
+  static const double from[2][8] = {{0, 4.6, 1.4, 0, 0, 0, 0, 0}, {0, 11.3, 7.8, 5.5, 0.8, 0, 0, 0}};
   const double n = L.np, cells = (double)L.nc[0] * L.nc[1] * (L.dim == 3 ? L.nc[2] : 1);
   const double fma = L.dim == 2 ? n * (4 * n * n + 4 * (2 * n + 2)) : n * n * (8 * n * n + 6 * (2 * n + 2));
   return cells * fma * 1.7e-6 >= from[L.dim - 2][L.k];
