@@ -200,7 +200,7 @@ int tpss_precond_create(const tpss_layout *layout, tpss_operator *op,
 int tpss_precond_create_shallow(const tpss_precond *other, const tpss_precond_desc *desc,
                                 tpss_precond **out);
 /* SchwarzPreconditioner::vmult (schwarz_preconditioner.templates.h:209-239): dst is set to
- * zero and receives sum over colors of omega R_j^T A_j^-1 R_j src.  FP64, additive vertex patches on a
+ * zero and receives sum over colors of omega R_j^T A_j^-1 R_j src.  FP64, additive vertex patches (two and more) on a
  * Cartesian level: the handle (a shallow copy too) holds intermediate vectors, 10 values per DoF
  * in 3D and 4 in 2D, allocated when it is created; without room for them then it applies the
  * patches color by color (1.7 times the time).  These applications allocate nothing. */

@@ -780,15 +780,17 @@ bool use_stream(const tpss_precond *p)
 
 namespace
 {
-// the direction-by-direction FP64 smoother applies: additive vertex patches of a Cartesian level
-// with keyed fast-diagonalization tables and at least one patch
+// The direction-by-direction FP64 smoother applies: additive vertex patches of a Cartesian level
+// with keyed fast-diagonalization tables. A level with a single patch shares nothing: the per-color kernel takes one launch
+// (2^3 cells, k = 1, 4, 7: 10.5, 15.2 and 28.6 us against 16.4, 24.6 and 34.9 for the five passes; 2^2 cells
+// equal). With two patches the passes are ahead or equal (2 x 2 x 3, k = 1, 4, 7: 18.9, 31.4, 47.5 against 20.6, 32.3, 64.5).
 bool sweep_eligible(const tpss_precond *p)
 {
   const tpss_layout &L = *p->tables->layout;
   if(p->desc.precision != TPSS_FP64 || p->desc.kernel_variant != TPSS_KERNEL_AUTO) return false;
   if(L.smoother_variant != TPSS_ADDITIVE || L.patch_variant != TPSS_PATCH_VERTEX || L.per_patch_fd) return false;
   if(p->tables->dense || p->tables->own_fd.n || p->tables->rcp_E < 0 || p->desc.use_ras_boolean_weights) return false;
-  return L.P > 0 && !L.vertex_fd[0].empty();
+  return L.P > 1 && !L.vertex_fd[0].empty();
 }
 
 // line arrays of the sweep: values per array (T1 / U1, T2, U2; 2D: T1, U1)
