@@ -793,13 +793,15 @@ bool sweep_eligible(const tpss_precond *p)
   return L.P > 1 && !L.vertex_fd[0].empty();
 }
 
-// line arrays of the sweep: values per array (T1 / U1, T2, U2; 2D: T1, U1)
+// line arrays of the sweep: values per array (T1 / U1, T2, U2; 2D: T1, U1), each beginning on a 256-byte boundary of
+// their one allocation
 std::array<size_t, 3> sweep_sizes(const tpss_layout &L)
 {
   const size_t mx = (size_t)(L.nc[0] - 1) * L.n, gy = (size_t)L.nc[1] * L.np;
-  if(L.dim == 2) return {mx * gy, mx * gy, 0};
+  auto pad = [](size_t n) { return (n + 31) / 32 * 32; };
+  if(L.dim == 2) return {pad(mx * gy), pad(mx * gy), 0};
   const size_t my = (size_t)(L.nc[1] - 1) * L.n, gz = (size_t)L.nc[2] * L.np;
-  return {mx * gy * gz, mx * my * gz, mx * my * gz};
+  return {pad(mx * gy * gz), pad(mx * my * gz), pad(mx * my * gz)};
 }
 
 // Line arrays of a new handle, where the sweep applies and the device has room for them (the per-color

@@ -174,16 +174,17 @@ void run(const tpss_operator &op, double *buf, double *dst, const double *src, c
     if constexpr(C::smem() > 48 * 1024)  // per device; a cheap host call
       TPSS_CUDA(cudaFuncSetAttribute(op_x_kernel<DIM, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem()));
     const int ng = L.nc[1] * (DIM == 3 ? L.nc[2] : 1);
-    // one-dimensional: a long level has more tiles along x than a grid's second dimension holds
-    const int64_t grid = (int64_t)((ng + C::XG - 1) / C::XG) * ((L.nc[0] + C::XC - 1) / C::XC);
-    op_x_kernel<DIM, N><<<(unsigned)grid, C::THREADS, C::smem(), s>>>(a);
+    // a long level has more tiles along x than a grid's second dimension holds: the third counts its multiples
+    const int tiles = (L.nc[0] + C::XC - 1) / C::XC;
+    const dim3 grid((ng + C::XG - 1) / C::XG, std::min(tiles, kMaxGridY), (tiles + kMaxGridY - 1) / kMaxGridY);
+    op_x_kernel<DIM, N><<<grid, C::THREADS, C::smem(), s>>>(a);
     TPSS_CUDA(cudaGetLastError());
   }
   auto line_launch = [&](auto mode, OpLineArgs a, int d) {
     // segments as for the smoother's lines (sweep64.cu): enough threads to fill the chip
     const int len = L.nc[d];
     int64_t segs = ((int64_t)num_sms() * 2048 + a.ncol - 1) / a.ncol;
-    segs = std::min<int64_t>(std::max<int64_t>(segs, 1), std::min(len, kMaxSegments));
+    segs = std::min<int64_t>(std::max<int64_t>(segs, 1), std::min(len, kMaxGridY));
     a.seg = (int)((len + segs - 1) / segs);
     const dim3 grid((unsigned)((a.ncol + kOpThreads - 1) / kOpThreads), (unsigned)((len + a.seg - 1) / a.seg));
     op_line_kernel<DIM, N, decltype(mode)::value><<<grid, kOpThreads, 0, s>>>(a);

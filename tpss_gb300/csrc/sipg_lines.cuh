@@ -16,7 +16,7 @@
 // t+ = (sigma_b - 2 sigma) u - t; unequal widths shift t+ by the difference of the penalties.
 // All contractions run in even/odd form with integers, one exponent per pencil (fixed64.cuh).
 //
-// Measured, 64^3 cells, k = 4 (32.8M DoFs): 953 us (x 396, y 303, last 252) against sipg_kernel's
+// Measured, 64^3 cells, k = 4 (32.8M DoFs): 940 us (x 382, y 303, last 252) against sipg_kernel's
 // 3,168 us, whose FP64 pipe is busy throughout. The vectors in between cost 2.4 GB of traffic in all
 // (0.36 ms at the copy rate), which the cell-wise kernel does not have; issue slots (56 % busy) and the
 // 32-bit multiplier (46 to 55 %) bound the passes. Of the conversions back to FP64 the results' use the
@@ -112,7 +112,7 @@ __device__ __forceinline__ void split_parts(const double (&u)[N], int emax, int 
 // which do not depend on it, any bits, nor makes them differ between a cell and its copy at the end of a tile
 // or segment. A face value more than two binades above q enters r in FP64 instead; it is rare and read once more
 // there (again: sets uL, uR), since the registers that would keep it cost 15 % of the passes' time (64^3 cells, k = 4:
-// 1,106 us; 953 so; 903 with one unit for q and the face values).
+// 1,106 us; 940 so; 903 with one unit for q and the face values).
 template<int N, bool HAS_P, bool WANT_M, int PARTS, typename Again>
 __device__ __forceinline__ void cell_pencil(const int2 *__restrict__ tab, const double *__restrict__ tab64, int FM, int FC,
                                             int FT, const double (&p)[N], const double (&q)[N], double uL, double uR,
@@ -278,7 +278,7 @@ __device__ __forceinline__ void special_faces(const double *sg, bool below, bool
 
 // ---- y and last pass: one thread per line and segment
 constexpr int kOpThreads = 128;
-constexpr int kMaxSegments = 65535;  // a grid's second dimension (a longer line gets longer segments)
+constexpr int kMaxGridY = 65535;  // a grid's second dimension (a longer line gets longer segments)
 
 enum OpLineMode
 {
@@ -417,8 +417,8 @@ __global__ void __maxnreg__((x_regs(N))) op_x_kernel(OpLineArgs a)
   double *s_r = s_tr + 2 * P, *s_m = s_r + N * CS;
   int64_t *s_row = reinterpret_cast<int64_t *>(s_m + N * CS);
   const int tid = threadIdx.x, lane = tid % 32, warp = tid / 32, nx = a.nc[0];
-  const int ng = a.nc[1] * (DIM == 3 ? a.nc[2] : 1), groups = (ng + C::XG - 1) / C::XG;
-  const int g0 = blockIdx.x % groups * C::XG, x0 = blockIdx.x / groups * XC;
+  const int ng = a.nc[1] * (DIM == 3 ? a.nc[2] : 1), g0 = blockIdx.x * C::XG, x0 = (blockIdx.y + blockIdx.z * kMaxGridY) * XC;
+  if(x0 >= nx) return;  // (all threads: the last multiple of the second dimension is not full)
   const int64_t gx_n = (int64_t)nx * N;
   const int w0 = a.width[x0] & ~kSpecial;
   // one table serves the tile when its cells have the same width

@@ -23,9 +23,10 @@ void launch_x(const XArgs &a, cudaStream_t s)
     TPSS_CUDA(cudaFuncSetAttribute(sweep_x_kernel<DIM, K1, FWD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)C::smem()));
   const int per = FWD ? C::XV : C::XV - 1, count = FWD ? a.nx - 1 : a.nx;
-  // one-dimensional: a long level has more tiles along x than a grid's second dimension holds
-  const int64_t grid = (int64_t)((a.ny * a.nz + C::XG - 1) / C::XG) * ((count + per - 1) / per);
-  sweep_x_kernel<DIM, K1, FWD><<<(unsigned)grid, C::THREADS, C::smem(), s>>>(a);
+  // a long level has more tiles along x than a grid's second dimension holds: the third counts its multiples
+  const int tiles = (count + per - 1) / per;
+  const dim3 grid((a.ny * a.nz + C::XG - 1) / C::XG, tiles < kMaxGridY ? tiles : kMaxGridY, (tiles + kMaxGridY - 1) / kMaxGridY);
+  sweep_x_kernel<DIM, K1, FWD><<<grid, C::THREADS, C::smem(), s>>>(a);
   TPSS_CUDA(cudaGetLastError());
 }
 
@@ -39,7 +40,7 @@ void launch_line(LineArgs a, cudaStream_t s)
   const int64_t want = (int64_t)num_sms() * 2048;
   int64_t segs = (want + a.ncol - 1) / a.ncol;
   if(segs > len) segs = len;
-  if(segs > kMaxSegments) segs = kMaxSegments;
+  if(segs > kMaxGridY) segs = kMaxGridY;
   if(segs < 1) segs = 1;
   a.seg = (int)((len + segs - 1) / segs);
   const dim3 grid((unsigned)((a.ncol + kLineThreads - 1) / kLineThreads), (unsigned)((len + a.seg - 1) / a.seg));

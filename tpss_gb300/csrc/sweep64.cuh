@@ -39,7 +39,7 @@ using fd::Entry;
 using fd::EoEntry;
 
 constexpr int kLineThreads = 128;
-constexpr int kMaxSegments = 65535;  // a grid's second dimension (a longer line gets longer segments)
+constexpr int kMaxGridY = 65535;  // a grid's second dimension (a longer line gets longer segments)
 
 struct SweepTab
 {
@@ -305,10 +305,10 @@ __global__ void __launch_bounds__(XCfg<DIM, K1>::THREADS) sweep_x_kernel(XArgs a
   int64_t *s_col = sx + XV * ES;
   double *s_cold = reinterpret_cast<double *>(s_col);
   int64_t *s_row = s_col + N * CS;  // first value of each row, -1 beyond the last cell row
-  const int tid = threadIdx.x, lane = tid % 32, warp = tid / 32, ng = a.ny * a.nz, groups = (ng + XG - 1) / XG;
-  const int g0 = blockIdx.x % groups * XG;
+  const int tid = threadIdx.x, lane = tid % 32, warp = tid / 32, ng = a.ny * a.nz, g0 = blockIdx.x * XG;
   // forward: vertices 1 + XV t ..; backward: the cells [x0, x0 + XV - 1) and the vertices around them
-  const int x0 = blockIdx.x / groups * (FWD ? XV : XV - 1);
+  const int x0 = (blockIdx.y + blockIdx.z * kMaxGridY) * (FWD ? XV : XV - 1);
+  if(x0 >= (FWD ? a.nx - 1 : a.nx)) return;  // (all threads: the last multiple of the second dimension is not full)
   const int vfirst = FWD ? x0 + 1 : x0;
   for(int s = 0; s < XV; ++s)
   {
