@@ -142,7 +142,7 @@ int tpss_operator_create_penalty(const tpss_layout *layout, double ip_factor, in
 /* MF::Operator::vmult (apps/laplace_integrator.h:578-598), FP64.  On Cartesian levels but the
  * smallest the operator holds intermediate vectors for it, 4 values per DoF in 3D and 2 in 2D, allocated
  * when it is created; without room for them then it uses a kernel that needs none (3D DGQ4:
- * 3.3 times the time).  A product allocates nothing. */
+ * 3.4 times the time).  A product allocates nothing. */
 int tpss_operator_vmult(tpss_operator *op, double *dst, const double *src, void *stream);
 /* The same product in FP32 arithmetic on FP64 vectors (src is converted once into a scratch
  * copy owned by the operator; dst is written in FP64): the level operator of a single-precision
